@@ -205,3 +205,27 @@ def tolerance(case: dict):
     if case["op"] in ("load", "pack", "unpack", "embed"):
         return "exact"
     return {"rel": 1.2e-3, "max": 3.1e-2}
+
+
+def exact(case: dict, seed: int):
+    """What `run` gives, in 64 bits from the dense weights; packed arrays have no such value."""
+    op, g = case["op"], _gen(seed, 0)
+    if op == "linear":
+        w, x = _weight((case["out"], case["in"]), g), _x(case["rows"], case["in"], g)
+        return x.double() @ w.double().T
+    if op == "layer":
+        ws = {name: _weight(shape, g) for name, shape in _layer_shapes(case).items()}
+        q, o, f, d = (_x(1, k, g).double() for k in (case["hidden"], case["q"], case["hidden"], case["ffn"]))
+        return [x @ ws[name].double().T for name, x in (("q", q), ("k", q), ("v", q), ("o", o), ("gate", f), ("up", f), ("down", d))]
+    if op == "moe":
+        e, n, d, top = case["experts"], case["n"], case["hidden"], case["top"]
+        gate_up, down = _weight((e, 2 * n, d), g), _weight((e, d, n), g)
+        x = _x(case["tokens"], d, g).double()
+        experts = torch.rand((case["tokens"], e), generator=g, device="cuda").topk(top).indices
+        y = torch.empty((case["tokens"], top, d), dtype=torch.float64, device="cuda")
+        for i in experts.unique().tolist():
+            token, slot = torch.nonzero(experts == i, as_tuple=True)
+            gate, up = (x[token] @ gate_up[i].double().T).chunk(2, dim=1)
+            y[token, slot] = (torch.nn.functional.silu(gate) * up) @ down[i].double().T
+        return y
+    return None
