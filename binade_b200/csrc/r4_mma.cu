@@ -9,10 +9,10 @@
 // One block per SM, each with an equal share of the weight rows; one warp issues the TMA copies
 // and the MMAs; a ring of stages (mbarriers: `full` armed by the decoders and the TMA bytes,
 // `empty` by tcgen05.commit) lets decode run ahead. Two decode sides:
-//   r4_mma_oct_kernel  up to 128 input rows, K % 16 == 0: 26 warps, eight threads per weight row,
-//                      private cp.async rings (the batch-1 matvec's decode, oct.cuh)
-//   r4_mma_kernel      the rest: 14 warps, a warp per row and stage, 8 rows each, raw bytes and
-//                      codes fetched two stages ahead into registers
+//   r4_mma_oct_kernel  K % 16 == 0: up to 26 warps, eight threads per weight row, private
+//                      cp.async rings (the batch-1 matvec's decode, oct.cuh)
+//   r4_mma_kernel      the rest (many input rows with many weight rows a block, where the other's
+//                      stages do not fit; K % 16 == 8; unaligned arrays): 14 warps, a warp per row and stage, 8 rows each, raw bytes and codes fetched two stages ahead into registers
 // The weights are read once whatever M. The sum over K is the hardware's: 16 k per MMA step, in
 // order, from zero, in fp32: not the documented lane order of the one-row kernels, but the
 // order of cuBLAS's BF16 GEMM on this GPU, whose outputs this kernel reproduces bit for bit;
@@ -37,6 +37,8 @@ constexpr int MMA_OCT_WARPS = 26;     // decode warps of the eight-threads-per-r
 constexpr int MMA_BM = 128;                  // MMA M: rows of the A tile (the block's rows, then unused)
 constexpr int MMA_BK = 128;                  // k per stage: one R4 tile
 constexpr uint32_t MMA_A_STAGE = MMA_BM * MMA_BK * 2;  // 32 KB: two 64-k atoms of 128 rows x 128 B
+constexpr int MMA_RING = 2;            // tiles in a decode warp's ring: 2 / 3 / 4 measured 33.0 / 36.7 / 37.1 us (15360 x 3840, 17 input rows) and 66.5 / 70.9 / 70.9 us (3840 x 15360, 128): stages are worth more than ring slots
+constexpr uint32_t MMA_BARS = 256;           // bytes of the eight-threads-per-row kernel's barriers: two rings of at most eight slots, `done`, the TMEM address
 constexpr uint32_t MMA_SPIN_LIMIT = 1u << 22;
 constexpr uint32_t MMA_SMEM_MAX = 226 * 1024;  // dynamic part; the pair-table builder keeps 64 static bytes
 
@@ -70,6 +72,30 @@ __device__ __forceinline__ bool mm_bar_wait(uint32_t bar, uint32_t parity) {
   }
   atomicExch(&g_mma_error, 1);
   return false;
+}
+// Whether the phase is over already; does not wait.
+__device__ __forceinline__ bool mm_bar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// True in one lane of the (converged) warp. Instructions that a single thread issues (MMAs, commits,
+// bulk copies) take their operands from uniform registers; behind `lane == 0` the compiler has to
+// assume divergent values and wraps each of them in code that makes them uniform.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -171,10 +197,10 @@ __device__ __forceinline__ bool mma_issue_side(const CUtensorMap *x_map, const M
 
 // Warps 0..3: accumulators out of tensor memory (TMEM lane = weight row of the block), rounded to
 // BF16 and stored.
-__device__ __forceinline__ void mma_store_side(const MmaArgs &a, const MmaWindow &m, uint32_t tmem, uint32_t warp, uint32_t lane, int64_t row_base, int rows, bool ok) {
+__device__ __forceinline__ void mma_store_side(const MmaArgs &a, const MmaWindow &m, uint32_t tmem, uint32_t warp, uint32_t lane, int64_t row_base, int rows, bool ok, int mma_m = MMA_BM) {
   if (ok) ok = mm_bar_wait(m.done, 0);
   tc_fence_after();
-  const int r = (int)(warp * 32 + lane);
+  const int r = mma_m == 64 ? (lane < 16 ? (int)(warp * 16 + lane) : MMA_BM) : (int)(warp * 32 + lane);  // M = 64: 16 rows in the lower half of each warp's lanes
   if (!ok) return;
   if (a.split == 1) {  // the common case, kept free of the slice loop
     for (int c = 0; c < a.BN; c += 8) {
@@ -326,66 +352,130 @@ __global__ void __launch_bounds__((DW + 1) * 32, 1) r4_mma_kernel(const __grid_c
 // rows per warp, up to 26 decode warps = 104 rows per block, every thread streaming its own bytes
 // through a private cp.async ring of D tiles. About half the instructions per weight of the
 // kernel above (one 16-byte and one 8-byte shared load bring what eight 4-byte and 2-byte global
-// loads brought; the escape patch runs once per four rows), which is what bounds both. Takes
-// M <= 128 (the rings need the shared memory that wider B stages would use) and K % 16 == 0.
-template <int MAXW, int D, bool COLS>
-__global__ void __launch_bounds__((MAXW + 1) * 32, 1) r4_mma_oct_kernel(const __grid_constant__ CUtensorMap x_map, MmaArgs a) {
+// loads brought; the escape patch runs once per four rows). Takes K % 16 == 0, and M as far as two
+// stages fit beside the rings (104 rows a block: M <= 176; few rows: any).
+//
+// What bounds it: with 104 rows a block, the instructions of the decode; with few rows a block the
+// latency of one tile's chain in a warp (copy wait, table, patch, stage wait, proxy fence: 1500
+// to 1900 cycles), which seven warps cannot hide, and then the MMA warp (an MMA reads its A rows
+// from shared memory: 59 cycles with M = 128, whatever N up to 128). So:
+//   phases    the block's warps are dealt out to tile phases: the warps of phase f decode tiles
+//             f, f + phases, .. of their rows; the stages take the tiles in order, so sums keep the
+//             order of k. A thread's escape cursors still have to pass the tiles of the other
+//             phases; only code words of tiles that its row flags matter for that, and those
+//             are copied into the ring and counted
+//   A stages  hold the block's rows only: the MMA reads its M rows from their start, the rest of
+//             which are other stages' bytes and end in accumulator lanes that nobody reads (the
+//             window goes on past the last stage). Smaller stages mean more of them
+//   M = 64    for blocks of up to 64 rows
+//   MMA warp  issues through elect.sync and asks for the next stage before it issues (waiting
+//             stages and uniform operands took 1000 of 1500 cycles a tile)
+// Measured (us, before -> now): 3840 rows out of 15360 columns 129 -> 51 at 17 input rows, 148 -> 67
+// at 128, 133 -> 92 at 200; 15360 rows out of 3840 columns 37.9 -> 33.0, 43.8 -> 44.4, 50.8 -> 50.3.
+struct MmaOctPlan {
+  int phases, groups;   // tile phases; row groups of four (groups * phases decode warps)
+  int a_rows;           // rows of an A stage: the block's, rounded up to 8
+  int m;                // MMA M: 64 for up to 64 rows (half the A bytes to read per MMA, which is what few input rows cost), else 128
+  int slots;            // stages
+  uint32_t ring_slot;   // bytes of a warp's ring slot: 512 raw, 256 codes, 256 for the codes of each skipped tile
+  uint32_t flag_words;  // words of a row's flag bits in shared memory, a zero word in front
+};
+
+// Passes `n` escapes of a column that other warps apply.
+__device__ __forceinline__ void stream_skip(uint32_t n, EscStream &e, const uint8_t *__restrict__ esc_cols) {
+  const uint32_t q = e.q + n;
+  if ((q ^ e.q) >> 2) e.word = __ldg(reinterpret_cast<const uint32_t *>(esc_cols + (q & ~3u)));
+  e.q = q;
+}
+
+// PHASED: more than one tile phase (column-ordered escapes only).
+template <int MAXW, int D, bool COLS, bool PHASED>
+__global__ void __launch_bounds__((MAXW + 2) * 32, 1) r4_mma_oct_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ MmaArgs a, const __grid_constant__ MmaOctPlan pl) {
   constexpr int R = 4;
   using Geo = OctGeom<R>;
-  constexpr uint32_t SLOT = Geo::SLOT, RING = D * SLOT;
   extern __shared__ uint8_t mma_smem[];
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  const int T = a.T, S = a.stages, BN = a.BN;
+  const int T = a.T, S = a.stages, P = PHASED ? pl.phases : 1;
   const int64_t K = a.K;
-  const uint32_t b_stage = (uint32_t)BN * MMA_BK * 2u;
-  // shared window: A stages | B stages | pair table | barriers | rings
+  const uint32_t a_atom = (uint32_t)pl.a_rows * 128u, a_stage = 2u * a_atom, b_atom = (uint32_t)a.BN * 128u, b_stage = 2u * b_atom;
+  // shared window: A stages | B stages | pair table | barriers | flag bits | rings
   const uint32_t base = (smem_addr(mma_smem) + 1023u) & ~1023u;
-  const uint32_t a_at = base, b_at = a_at + (uint32_t)S * MMA_A_STAGE, lut_at = b_at + (uint32_t)S * b_stage;
-  const uint32_t bar_at = lut_at + LUT_WORDS * 4u, ring_at = bar_at + 256u;
+  const uint32_t a_at = base, b_at = a_at + (uint32_t)S * a_stage, lut_at = b_at + (uint32_t)S * b_stage;
+  const uint32_t bar_at = lut_at + LUT_WORDS * 4u, flag_at = bar_at + MMA_BARS, ring_at = (flag_at + (PHASED ? (uint32_t)a.rows * pl.flag_words * 4u : 0u) + 127u) & ~127u;
   const MmaWindow win{a_at, b_at, b_stage, bar_at, bar_at + 8u * S, bar_at + 16u * S, bar_at + 16u * S + 8u};
   uint8_t *const gen = mma_smem + (base - smem_addr(mma_smem));
 
   const int64_t row_base = (int64_t)blockIdx.x * a.rows;
   const int rows = (int)min((int64_t)a.rows, a.N - row_base);
-  const uint32_t active = (uint32_t)(rows + R - 1) / R;  // decode warps with rows
+  const uint32_t decoders = (uint32_t)(pl.groups * P);
+  const uint32_t active = (uint32_t)(rows + R - 1) / R;  // row groups with rows in this block
+  const uint32_t group = warp % (uint32_t)pl.groups, phase = warp / (uint32_t)pl.groups;
+  const bool decoder = warp < decoders && group < active, mma_warp = warp == decoders, x_warp = warp == decoders + 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) mm_bar_init(win.full + 8 * s, active + 1), mm_bar_init(win.empty + 8 * s, 1);
     mm_bar_init(win.done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == MAXW) {
+  if (mma_warp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(win.slot), "r"(a.tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
 
-  // ---- load side of a decode warp, started before the table is built
   const uint32_t grp = lane >> 3, p = lane & 7u;
-  const uint32_t r = warp * R + grp;  // row of the A tile (and of the block)
-  const int64_t srow = row_base + min((int)r, rows - 1);  // a slot past the block's last row decodes that row again; its MMA row is never stored
-  const bool decoder = warp < active;
+  // ---- load side of a decode warp; with one phase it starts before the table is built
+  const uint32_t r = min(group * R + grp, (uint32_t)rows - 1u);  // a slot past the block's last row decodes that row again, into its own A row
+  const int64_t srow = row_base + r;
   const bool partial = (K & 127) != 0;
   const uint32_t pmax = (uint32_t)(K & 127) / 16u;  // threads that hold weights in a short last tile
-  const uint32_t ring = ring_at + warp * RING + lane * 16u, to_codes = 512u - lane * 8u;
-  const uint8_t *praw = a.w.raw + srow * K + p * 16u;
-  const uint8_t *pcode = reinterpret_cast<const uint8_t *>(a.w.codes) + srow * ((int64_t)T * 64) + p * 8u;
-  int pt = 0;  // first tile the load side has not asked for
-  // the next tile into the slot at `at`, as one cp.async group (an empty group past the row's
-  // end, so that "all but the newest D - 1 groups" always names the tile being decoded); in a
-  // short last tile the threads past the row's end copy thread 0's bytes and ignore them
+  const uint32_t ring = ring_at + warp * (D * pl.ring_slot) + lane * 16u, to_codes = 512u - lane * 8u;
+  // the load side's next tile and this thread's bytes of it
+  int pt = (int)phase;
+  const uint8_t *raw = a.w.raw + srow * K + p * 16u + phase * 128u;
+  const uint8_t *code = reinterpret_cast<const uint8_t *>(a.w.codes) + srow * ((int64_t)T * 64) + p * 8u + phase * 64u;
+  const uint32_t my_flags = flag_at + r * pl.flag_words * 4u;
+  // bit 31: this thread's row flags tile t; bit 31 - i: tile t - i
+  auto flags_to = [&](int t) {
+    const uint32_t at = my_flags + ((uint32_t)t >> 5) * 4u;
+    return __funnelshift_l(lds_u32(at), lds_u32(at + 4u), 31u - ((uint32_t)t & 31u));
+  };
+  // the next tile into the slot at `at`, with the code words of the flagged tiles between this
+  // warp's previous tile and that one, as one cp.async group (an empty group past the row's end,
+  // so that "all but the newest D - 1 groups" always names the tile being decoded); in a short
+  // last tile the threads past the row's end copy thread 0's bytes and ignore them
   auto load_tile = [&](uint32_t at) {
     if (pt < T) {
       const bool tail = partial && pt == T - 1 && p >= pmax;
-      copy_tile<R, 0>(at, to_codes, tail ? praw - p * 16u : praw, pcode, true, 0.0f);
-      praw += 128, pcode += 64, pt++;
+      copy_tile<R, 0>(at, to_codes, tail ? raw - p * 16u : raw, code, true, 0.0f);
+      if constexpr (PHASED) {
+        uint32_t skipped = (flags_to(pt) << 1) >> (33 - P);  // bit i: tile pt - (P - 1) + i
+        while (skipped) {
+          const uint32_t i = 31u - (uint32_t)__clz((int)skipped);
+          skipped &= ~(1u << i);
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(at + to_codes + 256u + i * 256u), "l"(code - (P - 1 - (int)i) * 64) : "memory");
+        }
+      }
+      pt += P, raw += P * 128, code += P * 64;
     }
     cp_commit();
   };
-  if (decoder) {
+  const uint32_t slot_bytes = PHASED ? pl.ring_slot : 768u;
+  auto fill_ring = [&]() {
 #pragma unroll
-    for (int u = 0; u < D; u++) load_tile(ring + u * SLOT);
-  }
+    for (int u = 0; u < D; u++) load_tile(ring + u * slot_bytes);
+  };
 
+  if constexpr (PHASED) {  // flag bits of the block's rows, a zero word before each row's
+    uint32_t *const flag_words = reinterpret_cast<uint32_t *>(gen + (flag_at - base));
+    for (uint32_t i = warp; i < (uint32_t)rows * pl.flag_words; i += blockDim.x >> 5) {
+      const uint32_t row = i / pl.flag_words, w = i - row * pl.flag_words;
+      const int t = (int)(w * 32u + lane) - 32;
+      const uint32_t bits = __ballot_sync(BN_FULL, t >= 0 && t < T && a.w.flags[(row_base + row) * T + t] != 0);
+      if (lane == 0) flag_words[i] = bits;
+    }
+  } else if (decoder) {
+    fill_ring();
+  }
   build_pair_lut(reinterpret_cast<uint32_t *>(gen + (lut_at - base)), a.w.table);  // syncs once inside
   tc_fence_before();
   __syncthreads();
@@ -396,12 +486,12 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, 1) r4_mma_oct_kernel(const __
   bool ok = true;
 
   if (decoder) {
+    if constexpr (PHASED) fill_ring();
     OctSelf me;
     asm volatile("mov.u32 %0, 0;" : "=r"(me.ready)::"memory");  // after the barrier: orders the table reads
     me.lane = lane, me.lane_hi = lane & ~7u, me.to_codes = to_codes, me.lut = lut_at + lane * 4u;
     me.gmask = 0xFFu << (grp * 8u), me.ltg = me.gmask & lanemask_lt();
     me.esc = a.w.esc, me.esc_cap = a.w.n_esc + 1, me.esc_cols = a.w.esc_cols;
-    const uint8_t *const flags = a.w.flags + srow * T;
     uint32_t epos = __ldg(a.w.row_esc + srow);
     EscWindow ew{};
     EscStream col[2]{};  // with column-ordered escapes: this thread's columns 2p and 2p + 1
@@ -413,68 +503,127 @@ __global__ void __launch_bounds__((MAXW + 1) * 32, 1) r4_mma_oct_kernel(const __
       ew.base = epos & ~3u;
       ew.word = window_load(me.esc, me.esc_cap, ew.base + p * 4u);
     }
-    uint32_t nflag = p < 8u && (int)p < T ? (uint32_t)__ldg(flags + p) : 0u;  // this thread's flag byte of the next block of eight tiles
-    uint32_t fm = 0;
     // the two 16-byte chunks of this thread in a stage: k 16p .. 16p+7 and 16p+8 .. 16p+15 of row r
-    const uint32_t a_off0 = (p >> 2) * (MMA_BM * 128u) + swz(r, 2u * (p & 3u)), a_off1 = (p >> 2) * (MMA_BM * 128u) + swz(r, 2u * (p & 3u) + 1u);
-    int s = 0;
-    uint32_t ph = 1;  // parity of the `empty` phase that frees slot s (first pass: slots start free)
-    // D tiles a round, so that tile ct + u sits in slot u (an immediate offset)
-    for (int c0 = 0; c0 < T; c0 += D) {
+    const uint32_t a_off0 = a_at + (p >> 2) * a_atom + swz(r, 2u * (p & 3u)), a_off1 = a_at + (p >> 2) * a_atom + swz(r, 2u * (p & 3u) + 1u);
+    const uint8_t *const flags = a.w.flags + srow * T;
+    uint32_t nflag = !PHASED && (int)p < T ? (uint32_t)__ldg(flags + p) : 0u;  // this thread's flag byte of the next block of eight tiles
+    uint32_t fm = 0;
+    int s = (int)phase;  // A slot of tile t
+    uint32_t ph = 1;     // parity of the `empty` phase that frees it (first pass: slots start free)
+    while (s >= S) s -= S, ph ^= 1u;
+    // D tiles a round, so that their slots are fixed offsets of the ring
+    for (int t0 = (int)phase; t0 < T; t0 += D * P)
 #pragma unroll
-      for (int u = 0; u < D; u++) {
-        const int ct = c0 + u;
-        if (ct >= T) break;
-        const uint32_t at = ring + u * SLOT;
-        if ((ct & 7) == 0) {  // a new block of eight tiles: fold the flag bytes, fetch the next block's
+    for (int u = 0; u < D; u++) {
+      const int t = t0 + u * P;
+      if (t >= T) break;
+      const uint32_t at = ring + u * slot_bytes;
+      uint32_t fl = 0;  // bit 31: this thread's row flags the tile (one phase: a row of the warp does); below: the tiles before it
+      if constexpr (PHASED) {
+        fl = flags_to(t);
+      } else {
+        if ((t & 7) == 0) {  // a new block of eight tiles: fold the flag bytes, fetch the next block's
           const uint32_t v = __ballot_sync(BN_FULL, nflag != 0);
           fm = (v | (v >> 8) | (v >> 16) | (v >> 24)) & 0xFFu;
-          const int nt = ct + 8 + (int)p;
-          nflag = p < 8u && nt < T ? (uint32_t)__ldg(flags + nt) : 0u;
+          const int nt = t + 8 + (int)p;
+          nflag = nt < T ? (uint32_t)__ldg(flags + nt) : 0u;
         }
-        const uint32_t token = cp_wait<D - 1>();  // all but the newest D - 1 groups have landed: this tile's has
-        uint32_t rr[R], cc[Geo::NC], w[2 * R];
-        asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]) : "r"(at), "r"(token));
-        asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(cc[0]), "=r"(cc[1]) : "r"(at + to_codes), "r"(token));
+        fl = fm << (31 - (t & 7));
+      }
+      const uint32_t token = cp_wait<D - 1>();  // all but the newest D - 1 groups have landed: this tile's has
+      uint32_t rr[R], cc[Geo::NC], w[2 * R];
+      asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]) : "r"(at), "r"(token));
+      asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(cc[0]), "=r"(cc[1]) : "r"(at + to_codes), "r"(token));
 #pragma unroll
-        for (int i = 0; i < R; i++) {
-          const uint32_t c = (i & 1) ? cc[i >> 1] >> 16 : cc[i >> 1];
-          w[2 * i] = (__byte_perm(rr[i], 0u, 0x1100) & 0x807F807Fu) | lut_read(me.lut + ((c << 7) & 0x7F80u), me.ready);
-          w[2 * i + 1] = (__byte_perm(rr[i], 0u, 0x3322) & 0x807F807Fu) | lut_read(me.lut + ((c >> 1) & 0x7F80u), me.ready);
-        }
-        if ((fm >> (ct & 7)) & 1u) {
-          if constexpr (COLS) {
+      for (int i = 0; i < R; i++) {
+        const uint32_t c = (i & 1) ? cc[i >> 1] >> 16 : cc[i >> 1];
+        w[2 * i] = (__byte_perm(rr[i], 0u, 0x1100) & 0x807F807Fu) | lut_read(me.lut + ((c << 7) & 0x7F80u), me.ready);
+        w[2 * i + 1] = (__byte_perm(rr[i], 0u, 0x3322) & 0x807F807Fu) | lut_read(me.lut + ((c >> 1) & 0x7F80u), me.ready);
+      }
+      if constexpr (COLS) {
+        if (fl >> (32 - P)) {  // this row flags the tile or one that was skipped on the way to it
+          uint32_t skipped = PHASED ? (fl << 1) >> (33 - P) : 0u, n0 = 0, n1 = 0;
+          while (PHASED && skipped) {
+            const uint32_t i = 31u - (uint32_t)__clz((int)skipped);
+            skipped &= ~(1u << i);
+            uint32_t s0, s1;
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(s0), "=r"(s1) : "r"(at + to_codes + 256u + i * 256u), "r"(token) : "memory");
+            n0 += __popc(hits15(s0)), n1 += __popc(hits15(s1));
+          }
+          if (PHASED && n0) stream_skip(n0, col[0], a.w.esc_cols);
+          if (PHASED && n1) stream_skip(n1, col[1], a.w.esc_cols);
+          if (fl >> 31) {
             const uint32_t h0 = hits15(cc[0]), h1 = hits15(cc[1]);
             if (h0) stream_patch<0>(h0, col[0], a.w.esc_cols, w);
             if (h1) stream_patch<4>(h1, col[1], a.w.esc_cols, w);
-          } else {
-            oct_patch<R>(epos, ew, w, cc, me);
           }
         }
-        if (partial && ct == T - 1 && p >= pmax) {  // past the row's end: zeros (the columns of X there are zeros too, but 0 x Inf must not happen)
-#pragma unroll
-          for (int i = 0; i < 2 * R; i++) w[i] = 0u;
-        }
-        if (ct >= S && ok) ok = mm_bar_wait(win.empty + 8 * s, ph);
-        tc_fence_after();
-        const uint32_t a_s = a_at + (uint32_t)s * MMA_A_STAGE;
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a_s + a_off0), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a_s + a_off1), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-        fence_async_smem();  // the tensor core reads shared memory through the async proxy
-        __syncwarp();
-        if (lane == 0) mm_bar_arrive(win.full + 8 * s);
-        if (++s == S) s = 0, ph ^= 1u;
-        load_tile(at);  // the slot just read takes the tile D further on
+      } else {
+        if (fl >> 31) oct_patch<R>(epos, ew, w, cc, me);
       }
+      if (partial && t == T - 1 && p >= pmax) {  // past the row's end: zeros (the columns of X there are zeros too, but 0 x Inf must not happen)
+#pragma unroll
+        for (int i = 0; i < 2 * R; i++) w[i] = 0u;
+      }
+      if (t >= S && ok) ok = mm_bar_wait(win.empty + 8 * s, ph);
+      tc_fence_after();
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a_off0 + (uint32_t)s * a_stage), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a_off1 + (uint32_t)s * a_stage), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+      fence_async_smem();  // the tensor core reads shared memory through the async proxy
+      __syncwarp();
+      if (lane == 0) mm_bar_arrive(win.full + 8 * s);
+      s += P;
+      while (s >= S) s -= S, ph ^= 1u;
+      load_tile(at);  // the slot just read takes the warp's tile D further on
     }
     cp_wait<0>();
-  } else if (warp == MAXW) {
-    ok = mma_issue_side(&x_map, win, T, S, BN, a.slice_tiles, tmem, lane, ok);
+  } else if (mma_warp) {
+    const uint32_t idesc = mma_idesc(pl.m, a.BN);
+    int s = 0, in_slice = 0;  // slot of tile t, tile inside the current K slice
+    uint32_t ph = 0, acc = tmem;
+    // whether the next stage is there already: asked before the MMAs are issued (which takes as
+    // long as the tensor core needs for them), since the answer alone takes more than a hundred cycles
+    bool have = false;
+    for (int t = 0; t < T && ok; t++) {
+      if (!have) ok = mm_bar_wait(win.full + 8 * s, ph);
+      const int ns = s + 1 == S ? 0 : s + 1;
+      const uint32_t nph = ns ? ph : ph ^ 1u;
+      have = mm_bar_test(win.full + 8 * ns, nph);
+      tc_fence_after();
+      if (ok && elect_one()) {
+        const uint64_t da = smem_desc(a_at + (uint32_t)s * a_stage), db = smem_desc(b_at + (uint32_t)s * b_stage);
+#pragma unroll
+        for (int j = 0; j < MMA_BK / 16; j++)  // 16 k per MMA: 32 bytes further along the swizzled row (descriptors count 16 bytes)
+          mma_bf16(acc, da + ((j >> 2) * a_atom >> 4) + (j & 3) * 2, db + ((j >> 2) * b_atom >> 4) + (j & 3) * 2, idesc, (in_slice | j) != 0);
+        mma_commit(win.empty + 8 * s);  // arrives when these MMAs have read the stage
+      }
+      __syncwarp();
+      s = ns, ph = nph;
+      if (++in_slice == a.slice_tiles) in_slice = 0, acc += (uint32_t)a.BN;
+    }
+    if (ok && elect_one()) mma_commit(win.done);
+    __syncwarp();
+  } else if (x_warp) {
+    if (lane == 0) {  // X tiles: two boxes of 64 k
+      int s = 0;
+      uint32_t ph = 1;
+      for (int t = 0; t < T && ok; t++) {
+        if (t >= S) ok = mm_bar_wait(win.empty + 8 * s, ph);
+        if (!ok) break;
+        const uint32_t b_s = b_at + (uint32_t)s * b_stage;
+        mm_bar_expect_tx(win.full + 8 * s, b_stage);
+        tma_load_2d(b_s, &x_map, t * MMA_BK, 0, win.full + 8 * s);
+        tma_load_2d(b_s + b_atom, &x_map, t * MMA_BK + 64, 0, win.full + 8 * s);
+        if (++s == S) s = 0, ph ^= 1u;
+      }
+    }
+    __syncwarp();
   }
-  if (warp < 4) mma_store_side(a, win, tmem, warp, lane, row_base, rows, ok);
+  ok = __all_sync(BN_FULL, ok);
+  if (warp < 4) mma_store_side(a, win, tmem, warp, lane, row_base, rows, ok, pl.m);
   tc_fence_before();
   __syncthreads();
-  if (warp == MAXW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+  if (mma_warp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
 }
 
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -519,29 +668,38 @@ int mma_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int
   const cuuint32_t box[2] = {64, (cuuint32_t)a.BN}, elem[2] = {1, 1};
   if (encode(&x_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(x), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return fail(BN_ERR_CUDA, "cuTensorMapEncodeTiled failed for the input rows");
-  const uint32_t fixed = 1024 + LUT_WORDS * 4 + 256;  // alignment slack, pair table, barriers
-  const uint32_t per_stage = MMA_A_STAGE + (uint32_t)a.BN * MMA_BK * 2u;
-  // eight threads per row where the rings fit beside at least two stages
+  const uint32_t fixed = 1024 + LUT_WORDS * 4 + MMA_BARS;  // alignment slack, pair table, barriers
   if (K % 16 == 0 && !(((uintptr_t)w->raw | (uintptr_t)w->codes) & 15)) {
     constexpr int ow = MMA_OCT_WARPS;
+    const bool cols = w->esc_cols && w->col_esc && !(((uintptr_t)w->esc_cols | (uintptr_t)w->col_esc) & 3);
     int64_t rows = (N + mma_sms() - 1) / mma_sms();
     rows = (rows + 3) / 4 * 4;
     if (rows > ow * 4) rows = ow * 4;
-    a.rows = (int)rows;
-    const unsigned grid = (unsigned)((N + rows - 1) / rows);
-    for (int slots = 4; slots >= 3; slots--) {
-      const uint32_t rings = (uint32_t)ow * slots * 768u;
-      if (fixed + rings + 2 * per_stage > MMA_SMEM_MAX) continue;
-      int stages = (int)((MMA_SMEM_MAX - fixed - rings) / per_stage);
-      a.stages = stages > 4 ? 4 : stages;
-      const uint32_t smem = fixed + rings + (uint32_t)a.stages * per_stage;
-      const bool cols = w->esc_cols && w->col_esc && !(((uintptr_t)w->esc_cols | (uintptr_t)w->col_esc) & 3);
-      auto kern = slots == 4 ? (cols ? r4_mma_oct_kernel<ow, 4, true> : r4_mma_oct_kernel<ow, 4, false>) : (cols ? r4_mma_oct_kernel<ow, 3, true> : r4_mma_oct_kernel<ow, 3, false>);
+    MmaArgs b = a;
+    MmaOctPlan pl{};
+    b.rows = (int)rows, pl.groups = (int)rows / 4, pl.a_rows = (int)(rows + 7) / 8 * 8, pl.m = rows <= 64 ? 64 : MMA_BM;
+    pl.flag_words = (uint32_t)(a.T + 31) / 32 + 1;
+    const uint32_t stage = (uint32_t)(pl.a_rows + a.BN) * 256u;
+    // as many phases as the warps allow (at most four: every phase adds 256 bytes to a ring slot)
+    // with at least one stage more than phases. Measured with 1 / 2 / 3 phases (us): 28 rows a
+    // block, 15360 columns, 17 input rows 67.6 / 63.1 / 55.8; 16 rows a block, 3840 columns 21.1 /
+    // 18.2 / 16.2 (15.7 with four)
+    const int most = cols ? max(1, min(4, ow / pl.groups)) : 1;
+    for (int phases = most; phases >= 1; phases--) {
+      pl.phases = phases, pl.ring_slot = 512u + 256u * phases;
+      const uint32_t rings = (uint32_t)(pl.groups * phases * MMA_RING) * pl.ring_slot, flags = (phases > 1 ? (uint32_t)rows * pl.flag_words * 4u : 0u) + 128u;
+      const uint32_t left = fixed + flags + rings < MMA_SMEM_MAX ? MMA_SMEM_MAX - fixed - flags - rings : 0u;
+      b.stages = min(8, (int)(left / stage));
+      if (b.stages < (phases > 1 ? phases + 1 : 2)) continue;
+      const uint32_t smem = fixed + flags + rings + (uint32_t)b.stages * stage;
+      const unsigned grid = (unsigned)((N + rows - 1) / rows), threads = 32u * (unsigned)max(4, pl.groups * phases + 2);
+      auto kern = phases > 1 ? r4_mma_oct_kernel<ow, MMA_RING, true, true> : cols ? r4_mma_oct_kernel<ow, MMA_RING, true, false> : r4_mma_oct_kernel<ow, MMA_RING, false, false>;
       BN_CUDA(allow_smem(kern, smem));
-      kern<<<grid, (ow + 1) * 32, smem, s>>>(x_map, a);
+      kern<<<grid, threads, smem, s>>>(x_map, b, pl);
       return launched("r4_mma_oct_kernel");
     }
   }
+  const uint32_t per_stage = MMA_A_STAGE + (uint32_t)a.BN * MMA_BK * 2u;
   // an equal share of the rows for every SM, in whole warps' worth of rows
   constexpr int dw = MMA_DECODE_WARPS, rpw = MMA_RPW;
   int64_t rows = (N + mma_sms() - 1) / mma_sms();

@@ -715,6 +715,28 @@ def test_mma_decodes_every_weight(N, K, density):
                 break  # the big case: a few column blocks are enough
 
 
+@pytest.mark.parametrize("N,K,M,density", [(1, 656, 6, 0.05), (600, 640, 5, 0.3), (1900, 1296, 17, 0.002), (3840, 4112, 33, 0.01), (5000, 144, 100, 0.5), (9400, 1024, 64, 0.001), (700, 2064, 130, 0.1), (3700, 1296, 256, 0.003), (15360, 784, 200, 0.002)])
+def test_mma_tile_phases(N, K, M, density):
+    """Blocks with few weight rows deal their warps out to tile phases (four, three, two, one over
+    these row counts; MMAs of 64 and of 128 rows; X in one part and in two): the same bits as one
+    phase with row-ordered escapes gives, where no cursor has to pass a tile, and the fp32 product
+    (bound as in test_mma_rows_against_fp32)."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    w = torch.randn((N, K), generator=g, device="cuda") * 0.02
+    w = torch.where(torch.rand((N, K), generator=g, device="cuda") < density, w * 2**20, w).to(torch.bfloat16)
+    m = r4.R4Linear(r4.from_dense(w))
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    got = m.mma_rows(x, split=1)
+    plain = {k: v for k, v in m._a.items() if k not in ("esc_cols", "col_esc")}
+    assert np.array_equal(words(got), words(ck.r4_mma(plain, x, N, K)))
+    ref = x.double() @ w.double().T
+    bound = ref.abs() * 2.0**-7 + 2.0**-22 * K**0.5 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((got.double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("N,K", [(384, 1024), (520, 3840), (256, 15360), (128, 16384)])
 def test_mma_rows_in_the_order_of_cublas(N, K):
     """Split-K in the kernel (every slice from zero in its own accumulator, fp32 sums added in
