@@ -272,6 +272,35 @@ def test_transcode_many_rows(N, K, kind):
     assert np.array_equal(words(r4.R4Linear(a).dense()), u)
 
 
+@pytest.mark.parametrize("N,K", [(5, 4), (1, 128), (70, 132), (33, 2048), (9, 2052), (40, 4096), (11, 4100), (3, 12296), (1300, 260)])
+@pytest.mark.parametrize("kind", ["normal", "uniform", "long", "outliers"])
+def test_thread_per_tile_decode(N, K, kind):
+    """R4 arrays, BF16 rows and looked-up rows at the edges of the decoder with a thread per tile: 1,
+    2, 16, 17, 32, 33 and 97 tiles a row (several rows a warp, several chunks of a row), short last
+    tiles, every k, tiles longer than the scan's ring (qmax up to 63), many weights alive to the end."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+
+    rng = np.random.default_rng(N + K)
+    if kind == "uniform":
+        u = rng.integers(0, 1 << 16, (N, K)).astype(np.uint16)
+    elif kind == "long":  # exponents a weight apart in frequency: ranks up to 255 all over the tile
+        u = ((np.minimum(rng.geometric(0.02, (N, K)), 254) << 7) | rng.integers(0, 128, (N, K))).astype(np.uint16)
+    else:
+        u = weights(rng, (N, K), escapes=kind == "outliers")
+    p = packed_arrays(u)
+    a, want = r4.transcode(p), o.pack_r4(u)
+    for key in ("codes", "flags", "esc", "row_esc"):
+        assert np.array_equal(a[key].cpu().numpy().view(want[key].dtype).reshape(-1), want[key].reshape(-1)), key
+    d = {k: ck.to_device(p[k]) for k in ("raw", "table", "meta", "bits", "roff")}
+    out, rend = ck.rice_unpack(d["meta"].reshape(-1), d["bits"], d["roff"], d["table"], d["raw"], N, K)
+    assert np.array_equal(words(out), u)
+    assert np.array_equal(rend.cpu().numpy().view(np.uint32), np.append(p["roff"][1:], np.uint32(len(p["bits"]))))
+    ids = np.array([N - 1, 0, N, N // 2, 0], np.int32)
+    rows = words(ck.rice_lookup(d["meta"].reshape(-1), d["bits"], d["roff"], d["table"], d["raw"], N, K, ck.to_device(ids)))
+    assert np.array_equal(rows, np.where((ids < N)[:, None], u[np.minimum(ids, N - 1)], np.uint16(0)))
+
+
 def test_transcode_all_escapes_grows_scratch():
     """Uniform exponents: nearly every weight escapes, far beyond the default scratch size."""
     from binade_b200.cuda import r4
