@@ -35,6 +35,7 @@ _SIGNATURES = {
         "bn_r4_decode": [C.POINTER(R4Struct), _i64, _i64, _i64, _i64, _i64, _vp, _vp],
         "bn_r4_esc_columns": [C.POINTER(R4Struct), _i64, _i64, _vp, _vp, _vp],
         "bn_bf16_split_hist": [_vp, _i64, _vp, _vp, _vp],
+        "bn_rank_table": [_vp, _vp, _vp, _vp],
         "bn_rice_encode_plan": [_vp, _vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp],
         "bn_rice_encode_write": [_vp, _vp, _vp, _vp, _i64, _i64, _vp, _u64, _vp],
         "bn_r4_lookup": [C.POINTER(R4Struct), _i64, _vp, _i64, _i64, _vp, _vp],

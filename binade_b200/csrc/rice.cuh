@@ -37,6 +37,15 @@ struct RiceArgs {
   uint32_t *counters;
 };
 
+#ifdef __CUDACC__
+// The low n bits: all of them from 32 on, none below 1.
+__device__ __forceinline__ uint32_t low_mask(int n) {
+  uint32_t m;
+  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(m) : "r"((uint32_t)max(n, 0)));
+  return m;
+}
+#endif
+
 // Decode in two kernels, one thread per tile (rice_tiles.cu); -1 when the arrays are outside their
 // coverage. rice_tiles_r4 fills what rice_kernel<RICE_R4> fills, rice_tiles_unpack what
 // rice_kernel<RICE_UNPACK> fills.

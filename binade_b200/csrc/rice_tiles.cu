@@ -31,12 +31,6 @@ constexpr uint32_t SC_STRIDE = SC_RING + 12;         // the ring's first 12 word
 
 // Words outside [0, nwords) read as zero.
 __device__ __forceinline__ uint32_t word_at(const uint32_t *__restrict__ bits, uint64_t nwords, uint64_t i) { return i < nwords ? __ldg(bits + i) : 0u; }
-// The low n bits: all of them from 32 on, none below 1.
-__device__ __forceinline__ uint32_t low_mask(int n) {
-  uint32_t m;
-  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(m) : "r"((uint32_t)max(n, 0)));
-  return m;
-}
 // (hi:lo) >> n, n <= 32
 __device__ __forceinline__ void shift_out(uint32_t &lo, uint32_t &hi, uint32_t n) {
   lo = __funnelshift_rc(lo, hi, n);

@@ -104,16 +104,16 @@ def rice_encode_ranked(u: torch.Tensor, rank_d: torch.Tensor):
 def rice_encode(w: torch.Tensor) -> dict:
     """BF16 weights [.., K] on the device (bfloat16 or int16 words) -> the format-2 arrays as
     device tensors {"raw", "table", "meta", "bits", "roff", "shape"}, bit for bit what the host
-    packer writes (pack.pack). Two small host reads on the way: the exponent histogram (the rank
-    table is built on the host like the reference does) and the stream's length in words."""
-    from ..format import rank_table
-
+    packer writes (pack.pack). One small host read on the way: the stream's length in words."""
     shape = tuple(w.shape)
     u = w.contiguous().view(torch.int16).reshape(-1, shape[-1])
-    raw, hist = split_hist(u)
-    table, rank = rank_table(hist)
-    meta, bits, roff = rice_encode_ranked(u, to_device(rank))
-    return {"raw": raw.reshape(shape), "table": to_device(table), "meta": meta, "bits": bits, "roff": roff, "shape": shape}
+    raw = torch.empty(u.numel(), dtype=torch.uint8, device=u.device)
+    hist = torch.empty(256, dtype=torch.int32, device=u.device)
+    _call("bn_bf16_split_hist", _p(u), u.numel(), _p(raw), _p(hist))
+    table, rank = torch.empty(256, dtype=torch.uint8, device=u.device), torch.empty(256, dtype=torch.uint8, device=u.device)
+    _call("bn_rank_table", _p(hist), _p(table), _p(rank))
+    meta, bits, roff = rice_encode_ranked(u, rank)
+    return {"raw": raw.reshape(shape), "table": table, "meta": meta, "bits": bits, "roff": roff, "shape": shape}
 
 
 def rice_ranks(meta: torch.Tensor, bits: torch.Tensor, roff: torch.Tensor, K: int):

@@ -274,8 +274,8 @@ def test_transcode_many_rows(N, K, kind):
 
 @pytest.mark.parametrize("N,K", [(5, 4), (1, 128), (70, 132), (33, 2048), (9, 2052), (40, 4096), (11, 4100), (3, 12296), (1300, 260)])
 @pytest.mark.parametrize("kind", ["normal", "uniform", "long", "outliers"])
-def test_thread_per_tile_decode(N, K, kind):
-    """R4 arrays, BF16 rows and looked-up rows at the edges of the decoder with a thread per tile: 1,
+def test_thread_per_tile_codec(N, K, kind):
+    """File arrays, R4 arrays, BF16 rows and looked-up rows at the edges of the codec with a thread per tile: 1,
     2, 16, 17, 32, 33 and 97 tiles a row (several rows a warp, several chunks of a row), short last
     tiles, every k, tiles longer than the scan's ring (qmax up to 63), many weights alive to the end."""
     from binade_b200.cuda import kernels as ck
@@ -289,6 +289,9 @@ def test_thread_per_tile_decode(N, K, kind):
     else:
         u = weights(rng, (N, K), escapes=kind == "outliers")
     p = packed_arrays(u)
+    enc = ck.rice_encode(dev(u))
+    for key in ("raw", "table", "meta", "bits", "roff"):
+        assert np.array_equal(enc[key].cpu().numpy().view(p[key].dtype).reshape(-1), p[key].reshape(-1)), key
     a, want = r4.transcode(p), o.pack_r4(u)
     for key in ("codes", "flags", "esc", "row_esc"):
         assert np.array_equal(a[key].cpu().numpy().view(want[key].dtype).reshape(-1), want[key].reshape(-1)), key
