@@ -502,6 +502,7 @@ static int oct_launch_r(OctArgs &a, int64_t blocks, int64_t slots, cudaStream_t 
   int e = -1;
   if (R == 4) {
     if (warps <= 16 && e == -1) e = launch_oct_as<4, 2, 16>(a, (unsigned)blocks, (unsigned)slots, (unsigned)warps, s);
+    if (warps <= 24 && e == -1) e = launch_oct_as<4, 2, 24>(a, (unsigned)blocks, (unsigned)slots, (unsigned)warps, s);
     if (warps <= 26 && e == -1) e = launch_oct_as<4, 1, 26>(a, (unsigned)blocks, (unsigned)slots, (unsigned)warps, s);
     if (e == -1) e = launch_oct_as<4, 1, 32>(a, (unsigned)blocks, (unsigned)slots, (unsigned)warps, s);
   } else if (R == 2) {
