@@ -44,6 +44,13 @@ int oct_matvec_multi(const bn_r4 *const *w, const int64_t *N, uint16_t *const *y
 int oct_gather(const bn_r4 *w, const uint16_t *x, const uint32_t *xi, const uint32_t *ei, int64_t G, int64_t n, int64_t K, int64_t RS, int64_t R0, int64_t split, uint16_t *y, uint16_t *y2, cudaStream_t s);
 int oct_status(int *status);
 
+// 2..8 input rows, and the expert gather grouped by expert, in the same form (r4_oct_rows.cu); -1
+// when the shape is outside its coverage.
+int oct_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int64_t N, int64_t K, uint16_t *y, int64_t y_stride, cudaStream_t s);
+int oct_gather_grouped(const bn_r4 *w, const uint16_t *x, const uint32_t *xi, const uint32_t *seg, const uint32_t *order, int64_t E, int64_t G, int64_t n, int64_t K, int64_t RS, int64_t R0, int64_t split, uint16_t *y, uint16_t *y2, cudaStream_t s);
+int oct_rows_status(int *status);
+int oct_rows_status_reset();
+
 // Register-pipelined batch-1 matvec and expert gather (r4_direct.cu); -1 outside their coverage.
 int direct_matvec(const bn_r4 *w, const uint16_t *x, int64_t N, int64_t K, uint16_t *y, cudaStream_t s);
 int direct_gather(const bn_r4 *w, const uint16_t *x, const uint32_t *xi, const uint32_t *ei, int64_t G, int64_t n, int64_t K, int64_t RS, int64_t R0, int64_t split, uint16_t *y, uint16_t *y2, cudaStream_t s);

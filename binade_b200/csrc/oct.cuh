@@ -203,4 +203,39 @@ __device__ __forceinline__ void oct_patch(uint32_t &epos, EscWindow &win, uint32
   }
 }
 
+// acc += w.lo * x.lo; acc += w.hi * x.hi with BF16 factors widened exactly (two fused ops).
+__device__ __forceinline__ float fma2_bf16(uint32_t w, uint32_t x, float acc) {
+  asm("{\n\t.reg .b16 wl, wh, xl, xh;\n\t"
+      "mov.b32 {wl, wh}, %1;\n\t"
+      "mov.b32 {xl, xh}, %2;\n\t"
+      "fma.rn.f32.bf16 %0, wl, xl, %0;\n\t"
+      "fma.rn.f32.bf16 %0, wh, xh, %0;\n\t}"
+      : "+f"(acc)
+      : "r"(w), "r"(x));
+  return acc;
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// The shared window of the batch-1 kernels: the pair table on a 64 KB boundary (a lookup address is
+// one byte permute), rings below it and above.
+constexpr uint32_t OC_BASE_MAX = 2048;    // the dynamic shared window starts below this address
+constexpr uint32_t OC_LUT = 65536;        // absolute shared address of the pair table
+constexpr uint32_t OC_TOP = 131072;       // the table (and x) end here; rings sit below the table and above this
+constexpr uint32_t OC_SMEM_MAX = 227 * 1024 - 256;  // dynamic shared memory a block may ask for (the kernel also has 64 static bytes)
+
+// Where a block's rings sit in the shared window (absolute shared addresses; base = start of the
+// dynamic allocation): warps 0 .. in_a-1 below the table, the others above it.
+struct OctLayout {
+  uint32_t ring_a, in_a, end;
+};
+__host__ __device__ inline OctLayout oct_layout(uint32_t base, uint32_t warps, uint32_t ring) {
+  OctLayout L;
+  L.ring_a = (base + 127u) & ~127u;
+  L.in_a = (OC_LUT - L.ring_a) / ring;
+  if (L.in_a > warps) L.in_a = warps;
+  L.end = OC_TOP + (warps - L.in_a) * ring;
+  return L;
+}
+
 }  // namespace bn

@@ -33,11 +33,6 @@
 namespace bn {
 namespace {
 
-constexpr uint32_t OC_BASE_MAX = 2048;    // the dynamic shared window starts below this address
-constexpr uint32_t OC_LUT = 65536;        // absolute shared address of the pair table
-constexpr uint32_t OC_TOP = 131072;       // the table (and x) end here; rings sit below the table and above this
-constexpr uint32_t OC_SMEM_MAX = 227 * 1024 - 256;  // dynamic shared memory a block may ask for (the kernel also has 64 static bytes)
-
 // This thread's 4R values of x for tile U past xs: two BF16x2 words per lane word.
 template <int R, int U>
 __device__ __forceinline__ void x_read(uint32_t xs, uint32_t ready, uint32_t (&xx)[2 * R]) {
@@ -50,20 +45,6 @@ __device__ __forceinline__ void x_read(uint32_t xs, uint32_t ready, uint32_t (&x
     asm("ld.shared.v2.u32 {%0, %1}, [%2+%3];" : "=r"(xx[0]), "=r"(xx[1]) : "r"(xs), "n"(U * 512), "r"(ready));
   }
 }
-// acc += w.lo * x.lo; acc += w.hi * x.hi with BF16 factors widened exactly (two fused ops).
-__device__ __forceinline__ float fma2_bf16(uint32_t w, uint32_t x, float acc) {
-  asm("{\n\t.reg .b16 wl, wh, xl, xh;\n\t"
-      "mov.b32 {wl, wh}, %1;\n\t"
-      "mov.b32 {xl, xh}, %2;\n\t"
-      "fma.rn.f32.bf16 %0, wl, xl, %0;\n\t"
-      "fma.rn.f32.bf16 %0, wh, xh, %0;\n\t}"
-      : "+f"(acc)
-      : "r"(w), "r"(x));
-  return acc;
-}
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 constexpr int OC_MAT = 4;  // matrices that can share one launch (and one x)
 
 struct OctArgs {
@@ -85,20 +66,6 @@ struct OctArgs {
 };
 
 __device__ int g_oct_error;  // set when the shared window does not match the launch; read by bn_device_status()
-
-// Where a block's rings sit in the shared window (absolute shared addresses; base = start of the
-// dynamic allocation): warps 0 .. in_a-1 below the table, the others above it.
-struct OctLayout {
-  uint32_t ring_a, in_a, end;
-};
-__host__ __device__ inline OctLayout oct_layout(uint32_t base, uint32_t warps, uint32_t ring) {
-  OctLayout L;
-  L.ring_a = (base + 127u) & ~127u;
-  L.in_a = (OC_LUT - L.ring_a) / ring;
-  if (L.in_a > warps) L.in_a = warps;
-  L.end = OC_TOP + (warps - L.in_a) * ring;
-  return L;
-}
 
 // Per-thread state of the decode side.
 template <int R>

@@ -636,6 +636,7 @@ int stream_status_reset() {
 extern "C" int bn_device_status_reset(void) {
   if (int e = bn::stream_status_reset()) return e;
   if (int e = bn::oct_status_reset()) return e;
+  if (int e = bn::oct_rows_status_reset()) return e;
   if (int e = bn::mma_status_reset()) return e;
   return bn::exchange_status_reset();
 }
@@ -645,6 +646,8 @@ extern "C" int bn_device_status(int *status) {
   int stream = 0, mma = 0, xch = 0, oct = 0;
   BN_CUDA(cudaMemcpyFromSymbol(&stream, bn::g_stream_error, sizeof(int)));
   if (int e = bn::oct_status(&oct)) return e;
+  if (oct) stream |= 4;
+  if (int e = bn::oct_rows_status(&oct)) return e;
   if (oct) stream |= 4;
   if (int e = bn::mma_status(&mma)) return e;
   if (int e = bn::exchange_status(&xch)) return e;

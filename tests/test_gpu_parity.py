@@ -690,6 +690,23 @@ def test_small_m_rows(M):
     assert np.array_equal(words(got)[0], o.c_dense_rows(xw, u))
 
 
+@pytest.mark.parametrize("N,K,M", [(3996, 640, 2), (4001, 656, 3), (4100, 16384, 4), (4097, 15360, 3), (4096, 2816, 8), (8003, 1296, 7), (15392, 3840, 4), (20000, 1024, 5)])
+def test_rows_of_many_row_matrices(N, K, M):
+    """Two to eight input rows on matrices with enough rows for four rows a warp: x in the table's
+    free halves and above it, short last tiles, more input rows in the code than given, two passes
+    where x does not fit: the bits of the one-row kernel, row by row."""
+    from binade_b200.cuda import r4
+
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    w = torch.randn((N, K), generator=g, device="cuda") * 0.02
+    w = torch.where(torch.rand((N, K), generator=g, device="cuda") < 0.01, w * 64, w).to(torch.bfloat16)
+    m = r4.R4Linear(r4.from_dense(w))
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    got = words(m.fused_rows(x))
+    for i in range(M):
+        assert np.array_equal(got[i], words(m(x[i]))), i
+
+
 @pytest.mark.parametrize("M,N,K", [(16, 128, 128), (16, 256, 512), (32, 200, 3840), (128, 384, 1024), (24, 130, 264), (100, 96, 2048), (1, 64, 128), (256, 300, 768), (200, 1000, 1280), (300, 128, 256)])
 def test_mma_rows_against_fp32(M, N, K):
     """Tensor-core decode GEMM: the weights it multiplies by are exactly the decoded BF16 weights
