@@ -268,19 +268,46 @@ def r4_decode(a: dict, N: int, K: int, nb: int | None = None, rs: int | None = N
     return out
 
 
-def r4_gather_grouped(a: dict, x: torch.Tensor, xi: torch.Tensor, ei: torch.Tensor, E: int, max_per_expert: int, n: int, rs: int, r0: int, K: int, split: int | None = None):
+def route(indices: torch.Tensor, k: int, E: int, grouped: bool):
+    """The router's choices (int32 or int64, any shape, k a token) as slots, in one launch: (ei, xi,
+    rows, groups): int32 tensors with each slot's expert, its token and its own number, and with
+    grouped the pair (seg, order) of group_slots, else None."""
+    if indices.dtype not in (torch.int64, torch.int32):
+        indices = indices.to(torch.int64)
+    indices = indices.contiguous()
+    G = indices.numel()
+    ei, xi, rows = torch.empty((3, G), dtype=torch.int32, device=indices.device).unbind(0)
+    groups = (torch.empty(E + 1, dtype=torch.int32, device=indices.device), torch.empty(G, dtype=torch.int32, device=indices.device)) if grouped else None
+    _call("bn_moe_route", _p(indices), indices.dtype == torch.int64, G, k, E, _p(ei), _p(xi), _p(rows), *((_p(groups[0]), _p(groups[1])) if grouped else (None, None)))
+    return ei, xi, rows, groups
+
+
+def group_slots(ei: torch.Tensor, E: int):
+    """(seg [E + 1], order): expert e's slots are order[seg[e] : seg[e + 1]], for ei int32 [G]; ids
+    outside 0 .. E - 1 are in no group."""
+    seg = torch.empty(E + 1, dtype=torch.int32, device=ei.device)
+    order = torch.empty(ei.numel(), dtype=torch.int32, device=ei.device)
+    _call("bn_moe_route", _p(ei), 0, ei.numel(), 1, E, None, None, None, _p(seg), _p(order))
+    return seg, order
+
+
+def swiglu(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    """silu(gate) * up in fp32, rounded once to BF16 (bfloat16, contiguous, same shape)."""
+    h = torch.empty_like(gate)
+    _call("bn_swiglu", _p(gate), _p(up), gate.numel(), _p(h))
+    return h
+
+
+def r4_gather_grouped(a: dict, x: torch.Tensor, xi: torch.Tensor, ei: torch.Tensor, E: int, max_per_expert: int, n: int, rs: int, r0: int, K: int, split: int | None = None, groups=None):
     """r4_gather's outputs with every expert's rows read once for all its slots: the slots are
     sorted by expert on the device (no host sync) and each expert multiplies up to 8 input rows
     per pass. ei: int32 [G] expert of each slot (0 <= ei < E); max_per_expert bounds the slots of
     one expert (the token count when a token names an expert at most once). K % 16 == 0.
-    Slots whose expert id is NO_EXPERT (padding) sort behind every expert and are skipped."""
+    Slots whose expert id is NO_EXPERT (padding) are in no group and are skipped. groups: what
+    group_slots gave for these slots, when the caller has it."""
     G = ei.numel()
     dev = x.device
-    bucket = torch.clamp(ei.to(torch.int64) & 0xFFFFFFFF, max=E)  # padding slots: one bucket past the experts
-    order = torch.argsort(bucket, stable=True).to(torch.int32)
-    counts = torch.zeros(E + 1, dtype=torch.int32, device=dev).scatter_add_(0, bucket, torch.ones(G, dtype=torch.int32, device=dev))  # (bincount would synchronise)
-    seg = torch.zeros(E + 1, dtype=torch.int32, device=dev)
-    seg[1:] = torch.cumsum(counts[:E], 0).to(torch.int32)
+    seg, order = group_slots(ei, E) if groups is None else groups
     if split:
         y = torch.empty((G, split), dtype=torch.bfloat16, device=dev)
         y2 = torch.empty((G, n - split), dtype=torch.bfloat16, device=dev)

@@ -22,6 +22,8 @@ from __future__ import annotations
 import torch
 from torch import nn
 
+from . import kernels as ck
+
 
 def swiglu(up: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     """silu(gate) * up in fp32, rounded once to BF16 (the activation of Gemma/Llama style MoE)."""
@@ -47,27 +49,29 @@ class R4SwitchGLU(nn.Module):
         active expert's weights are read once (same bits as slot by slot); max_per_expert bounds
         the slots of one expert (default: the token count, right when a token names an expert at
         most once, as top-k routing does)."""
-        n, G = self.n, ei.numel()
-        rows = torch.arange(G, dtype=torch.int32, device=x.device)
-        if G >= self.GROUP_MIN_SLOTS * self.E:
-            cap = max_per_expert or x.shape[0]
-            gu = self._gu._gather_grouped(x, xi, ei, self.E, cap, 2 * n, 2 * n, split=n)
-            if gu is not None:
-                h = self._activation(gu[1], gu[0])
-                out = self._down._gather_grouped(h, rows, ei, self.E, cap, self.D, self.D)
-                if out is not None:
-                    return out
-        gate, up = self._gu._gather(x, xi, ei, 2 * n, 2 * n, split=n)
-        h = self._activation(up, gate)
-        return self._down._gather(h, rows, ei, self.D, self.D)
+        rows = torch.arange(ei.numel(), dtype=torch.int32, device=x.device)
+        ei = ei.to(torch.int32).contiguous()
+        return self._run(x, xi, ei, rows, ck.group_slots(ei, self.E) if self._grouped(ei.numel()) else None, max_per_expert or x.shape[0])
+
+    def _grouped(self, G: int) -> bool:
+        return G >= self.GROUP_MIN_SLOTS * self.E and self.E <= 48 * 1024
+
+    def _run(self, x, xi, ei, rows, groups, cap: int) -> torch.Tensor:
+        n = self.n
+        gu = out = None
+        if groups is not None:
+            gu = self._gu._gather_grouped(x, xi, ei, self.E, cap, 2 * n, 2 * n, split=n, groups=groups)
+        gate, up = gu if gu is not None else self._gu._gather(x, xi, ei, 2 * n, 2 * n, split=n)
+        h = ck.swiglu(gate, up) if self._activation is swiglu else self._activation(up, gate)
+        if gu is not None:
+            out = self._down._gather_grouped(h, rows, ei, self.E, cap, self.D, self.D, groups=groups)
+        return out if out is not None else self._down._gather(h, rows, ei, self.D, self.D)
 
     def forward(self, x: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
         """x [..., D], indices [..., k] -> [..., k, D]."""
-        k = indices.shape[-1]
         flat = x.reshape(-1, x.shape[-1])
-        ei = indices.reshape(-1).to(torch.int32)
-        xi = torch.arange(ei.numel(), dtype=torch.int32, device=x.device) // k
-        return self.slots(flat, xi, ei).reshape(*indices.shape, self.D)
+        ei, xi, rows, groups = ck.route(indices.to(x.device), indices.shape[-1], self.E, self._grouped(indices.numel()))
+        return self._run(flat, xi, ei, rows, groups, flat.shape[0]).reshape(*indices.shape, self.D)
 
 
 class BinadeSwitchGLU(nn.Module):

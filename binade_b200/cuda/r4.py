@@ -158,12 +158,12 @@ class _R4:
         rows ei[g] * rs + r0 .. + n. With split, the pair [G, split], [G, n - split]."""
         return ck.r4_gather(self._a, x.contiguous(), xi.to(torch.int32), ei.reshape(-1).to(torch.int32), n, rs, r0, self.K, split, shape)
 
-    def _gather_grouped(self, x, xi, ei, E: int, max_per_expert: int, n: int, rs: int, r0: int = 0, *, split: int | None = None):
+    def _gather_grouped(self, x, xi, ei, E: int, max_per_expert: int, n: int, rs: int, r0: int = 0, *, split: int | None = None, groups=None):
         """_gather's outputs with every expert's rows read once for all the slots routed to it
         (bit-identical results); None when the shape is outside the grouped kernel (K % 16)."""
         if self.K % 16 or self.T > 200:
             return None
-        return ck.r4_gather_grouped(self._a, x.contiguous(), xi.to(torch.int32), ei.reshape(-1).to(torch.int32), E, max_per_expert, n, rs, r0, self.K, split)
+        return ck.r4_gather_grouped(self._a, x.contiguous(), xi.to(torch.int32), ei.reshape(-1).to(torch.int32), E, max_per_expert, n, rs, r0, self.K, split, groups)
 
     def dense(self, n: int | None = None, rs: int | None = None, r0: int = 0) -> torch.Tensor:
         """The BF16 weight, rebuilt from R4. With n, rs, r0: rows r0 .. r0 + n - 1 of every block of

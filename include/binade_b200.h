@@ -267,6 +267,17 @@ int bn_r4_gather_grouped(const uint16_t *x, const bn_r4 *w, const uint32_t *xi, 
                          int64_t n, int64_t K, int64_t RS, int64_t R0, int64_t split, uint16_t *y,
                          uint16_t *y2, void *stream);
 
+/* The router's choices as slots: ids [G] (int64 if ids64, else int32), k a token, in token order ->
+ * ei [G] expert, xi [G] = g / k, iota [G] = g; with seg [E+1] and order [G] the slots grouped by expert:
+ * expert e's are order[seg[e]] .. order[seg[e+1] - 1], in any order; ids outside 0 .. E-1 are in no
+ * group. Any output may be NULL (order goes with seg). E <= 49152 with seg. */
+int bn_moe_route(const void *ids, int ids64, int64_t G, int64_t k, int64_t E, uint32_t *ei, uint32_t *xi,
+                 uint32_t *iota, uint32_t *seg, uint32_t *order, void *stream);
+
+/* h [n] = silu(gate) * up (the activation between the gathers of an expert layer), BF16 in and out, in
+ * fp32 with one rounding. */
+int bn_swiglu(const uint16_t *gate, const uint16_t *up, int64_t n, uint16_t *h, void *stream);
+
 /* All-gather of small slices over NVLink peer memory, one kernel per rank (multi-GPU form of the
  * hook; the reference is single-device, so there is no counterpart). Every rank calls it with
  * 1..4 segments (one per projection): `locals[g]` is this rank's slice of segment g, `bytes[g]`

@@ -707,6 +707,52 @@ def test_rows_of_many_row_matrices(N, K, M):
         assert np.array_equal(got[i], words(m(x[i]))), i
 
 
+@pytest.mark.parametrize("E,n,D,tokens,topk", [(1, 704, 640, 2, 1), (8, 656, 1296, 5, 4), (33, 640, 704, 70, 3), (40, 704, 2816, 64, 8), (4, 1024, 4096, 90, 4), (3, 640, 16384, 9, 3)])
+def test_grouped_gather_shapes(E, n, D, tokens, topk):
+    """Slots grouped by expert (groups of four and of eight, half-filled groups, empty experts, padding
+    slots) against slot by slot, bit for bit, and the grouping itself."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+
+    g = torch.Generator(device="cuda").manual_seed(E * 7 + tokens)
+    w = torch.randn((E, 2 * n, D), generator=g, device="cuda") * 0.02
+    w = torch.where(torch.rand(w.shape, generator=g, device="cuda") < 0.002, w * 64, w).to(torch.bfloat16)
+    m = r4.R4Linear(r4.from_dense(w))
+    x = torch.randn((tokens, D), generator=g, device="cuda").to(torch.bfloat16)
+    ids = torch.rand((tokens, E), generator=g, device="cuda").topk(topk).indices
+    ids[tokens // 3] = -1
+    for dtype in (torch.int64, torch.int32):
+        ei, xi, rows, (seg, order) = ck.route(ids.to(dtype), topk, E, True)
+        assert torch.equal(ei, ids.reshape(-1).int()) and torch.equal(rows.cpu(), torch.arange(ei.numel(), dtype=torch.int32)) and torch.equal(xi, rows // topk)
+        s, h = seg.cpu().numpy(), order.cpu().numpy()
+        flat = ei.cpu().numpy()
+        for e in range(E):
+            assert np.array_equal(np.sort(h[s[e] : s[e + 1]]), np.flatnonzero(flat == e)), e
+        assert s[0] == 0 and s[E] == (flat >= 0).sum()
+    one = m._gather(x, xi, ei, 2 * n, 2 * n, split=n)
+    all_ = m._gather_grouped(x, xi, ei, E, tokens, 2 * n, 2 * n, split=n)
+    real = ei >= 0
+    for a, b in zip(one, all_):
+        assert np.array_equal(words(a[real]), words(b[real]))
+
+
+@pytest.mark.parametrize("n", [1, 2, 511, 513, 704 * 8])
+def test_swiglu_bits(n):
+    """The activation's kernel against torch's fp32 silu and product, bit for bit, infinities and NaN
+    among the values (NaN: any)."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import moe
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    gate, up = (torch.randn(n + 1, generator=g, device="cuda").mul_(8).to(torch.bfloat16) for _ in range(2))
+    gate[: min(n, 4)] = torch.tensor([float("inf"), float("-inf"), float("nan"), -100.0])[: min(n, 4)].to(torch.bfloat16)
+    for a, b in ((gate[:n], up[:n]), (gate[1:], up[1:])):  # the second: not 4-byte aligned
+        got, want = ck.swiglu(a, b), moe.swiglu(b, a)
+        assert torch.equal(got.isnan(), want.isnan())
+        keep = ~want.isnan()
+        assert np.array_equal(words(got[keep]), words(want[keep]))
+
+
 @pytest.mark.parametrize("M,N,K", [(16, 128, 128), (16, 256, 512), (32, 200, 3840), (128, 384, 1024), (24, 130, 264), (100, 96, 2048), (1, 64, 128), (256, 300, 768), (200, 1000, 1280), (300, 128, 256)])
 def test_mma_rows_against_fp32(M, N, K):
     """Tensor-core decode GEMM: the weights it multiplies by are exactly the decoded BF16 weights
