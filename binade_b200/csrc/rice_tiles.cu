@@ -290,6 +290,8 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
       const uint32_t *const slot = reinterpret_cast<const uint32_t *>(slots + (row + 1) * row_bytes) - T;
       const uint32_t w0 = a.roff[srow], begin = slot[t], end = t + 1 < T ? slot[t + 1] : begin + n * (k + qmax);
       const uint32_t first_word = w0 + (begin >> 5), last_word = w0 + (end >> 5);
+      // the raw bytes are only needed once the tiles are decoded: on their way to L2 meanwhile
+      if (MODE == RICE_UNPACK && mine) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.raw + srow * K + (int64_t)t * BN_TILE));
       __syncwarp();  // every entry of the chunk is read before anything is written
       uint32_t hits[4] = {0, 0, 0, 0}, low_at = 0, planes_at = 0, count = 0;
       for (int from = 0; from < tiles_here;) {
@@ -462,37 +464,47 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
         } else {
           // BF16 words: eight lanes a tile, sixteen weights a lane
           const bool wide = (K & 15) == 0;
-          for (int u0 = from; u0 < to; u0 += 4) {
+          // the raw bytes of step u0 (four tiles), one step ahead of their use
+          struct Piece {
+            int64_t row, col;
+            uint32_t rw[4];
+          };
+          auto fetch = [&](int u0) {
             const int u = u0 + (int)(lane >> 3);
             const int us = __shfl_sync(BN_FULL, sub, u & 31), ut = __shfl_sync(BN_FULL, t, u & 31);
-            const int64_t orow = row0 + us, irow = a.ids ? srow : orow;
-            const int64_t col = (int64_t)ut * BN_TILE + (lane & 7u) * 16;
-            if (u >= to || col >= K) continue;
-            const uint2 c = *reinterpret_cast<const uint2 *>(sc + u * TI_TILE + (lane & 7u) * 2);
-            const uint8_t *const raw = a.raw + irow * K + col;
-            uint32_t rw[4];
-            if (wide) {
+            Piece x{row0 + us, u < to ? (int64_t)ut * BN_TILE + (lane & 7u) * 16 : K, {0, 0, 0, 0}};
+            const uint8_t *const raw = a.raw + (a.ids ? srow : x.row) * K + x.col;
+            if (wide && x.col < K) {
               const uint4 v = __ldg(reinterpret_cast<const uint4 *>(raw));
-              rw[0] = v.x, rw[1] = v.y, rw[2] = v.z, rw[3] = v.w;
-            } else {
+              x.rw[0] = v.x, x.rw[1] = v.y, x.rw[2] = v.z, x.rw[3] = v.w;
+            } else if (x.col < K) {
 #pragma unroll
-              for (int i = 0; i < 4; i++) rw[i] = col + 4 * i < K ? ldg_stream_u32(raw + 4 * i) : 0u;
+              for (int i = 0; i < 4; i++)
+                if (x.col + 4 * i < K) x.rw[i] = ldg_stream_u32(raw + 4 * i);
             }
+            return x;
+          };
+          Piece next = fetch(from);
+          for (int u0 = from; u0 < to; u0 += 4) {
+            const Piece x = next;
+            if (u0 + 4 < to) next = fetch(u0 + 4);
+            if (x.col >= K) continue;
+            const uint2 c = *reinterpret_cast<const uint2 *>(sc + (u0 + (int)(lane >> 3)) * TI_TILE + (lane & 7u) * 2);
             uint32_t o[8];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
               const uint32_t cw = (i & 2 ? c.y : c.x) >> (16 * (i & 1));
-              o[2 * i] = (__byte_perm(rw[i], 0u, 0x1100) & 0x807F807Fu) | pair[cw & 0xFFu];
-              o[2 * i + 1] = (__byte_perm(rw[i], 0u, 0x3322) & 0x807F807Fu) | pair[(cw >> 8) & 0xFFu];
+              o[2 * i] = (__byte_perm(x.rw[i], 0u, 0x1100) & 0x807F807Fu) | pair[cw & 0xFFu];
+              o[2 * i + 1] = (__byte_perm(x.rw[i], 0u, 0x3322) & 0x807F807Fu) | pair[(cw >> 8) & 0xFFu];
             }
-            uint16_t *const dst = a.out + orow * K + col;
+            uint16_t *const dst = a.out + x.row * K + x.col;
             if (wide) {
               reinterpret_cast<uint4 *>(dst)[0] = make_uint4(o[0], o[1], o[2], o[3]);
               reinterpret_cast<uint4 *>(dst)[1] = make_uint4(o[4], o[5], o[6], o[7]);
             } else {
 #pragma unroll
               for (int i = 0; i < 4; i++)
-                if (col + 4 * i < K) *reinterpret_cast<uint2 *>(dst + 4 * i) = make_uint2(o[2 * i], o[2 * i + 1]);
+                if (x.col + 4 * i < K) *reinterpret_cast<uint2 *>(dst + 4 * i) = make_uint2(o[2 * i], o[2 * i + 1]);
             }
           }
           __syncwarp();  // the escaped weights' words are written over what went out above
