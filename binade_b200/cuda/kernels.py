@@ -28,6 +28,8 @@ def require_cuda() -> torch.device:
 
 def to_device(a, dtype=None) -> torch.Tensor:
     """numpy array or tensor -> contiguous CUDA tensor (uint16/uint32 travel as int16/int32)."""
+    if dtype is None and isinstance(a, torch.Tensor) and a.is_cuda and a.is_contiguous() and a.get_device() == torch.cuda.current_device():
+        return a  # the common case of arrays that are there already
     dev = require_cuda()
     if isinstance(a, np.ndarray):
         if a.dtype == np.uint16:
@@ -40,17 +42,26 @@ def to_device(a, dtype=None) -> torch.Tensor:
 
 
 def _p(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()  # (ctypes turns an int into the pointer argument)
 
 
 def _stream():
     """The current CUDA stream's handle (the raw query: building a torch Stream object per kernel
     call costs more host time than the launch)."""
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _call(fn, *args):
-    return _native.call("cuda", fn, *args, _stream())
+_entries: dict = {}  # entry points of the CUDA library by name
+
+
+def _call(name, *args):
+    fn = _entries.get(name)
+    if fn is None:
+        fn = _entries[name] = getattr(_native.load("cuda"), name)
+    status = fn(*args, _stream())
+    if status:
+        raise _native.NativeError(name, status, _native.load("cuda").bn_last_error().decode())
+    return status
 
 
 def r4_struct(a: dict) -> _native.R4Struct:
