@@ -27,13 +27,13 @@ from torch import nn
 from ..format import TILE
 from . import kernels as ck
 
-FUSED_MAX_ROWS = 4  # input rows served by the fused decode kernel in the documented order (15360 x 3840: 37 / 49 / 75 us at 2 / 4 / 8 rows); from 5 rows the tensor-core decode GEMM is faster (46 us)
+FUSED_MAX_ROWS = 4  # input rows served by the fused decode kernel in the documented order (15360 x 3840: 23 / 33 / 53 us at 2 / 4 / 8 rows); from 5 rows the tensor-core decode GEMM is faster (33 us)
 
 
 MMA_MAX_ROWS = 256  # input rows served by the tensor-core decode GEMM (one pass over the weights; 256 is the MMA's widest N); beyond, rebuild + cuBLAS
 
 
-MMA_MAX_PASSES = 1  # passes of MMA_MAX_ROWS rows that still beat rebuild + cuBLAS (15360 x 3840: 55 us a pass against 44 us for the rebuild: beyond one pass the rebuild wins)
+MMA_MAX_PASSES = 1  # passes of MMA_MAX_ROWS rows that still beat rebuild + cuBLAS (15360 x 3840: 50 us a pass of 200 rows against 46 us for the rebuild: beyond one pass the rebuild wins)
 
 
 class BinadeLinear(nn.Module):
