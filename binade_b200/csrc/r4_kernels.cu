@@ -415,7 +415,7 @@ extern "C" int bn_r4_rows(const uint16_t *x, int64_t x_stride, const bn_r4 *w, i
   cudaStream_t s = (cudaStream_t)stream;
   a.m = (int)M;
   // the instantiation is the next power of two >= M: absent input rows are zeros in shared
-  // memory and are never stored, so the weights stream once whatever M
+  // memory and are never stored
   if (M == 1) {
     // the cp.async kernel (K % 16 == 0, 640 <= K <= 16384, aligned arrays); else, for long rows,
     // the register-pipelined kernel; else the bulk-copy kernel (K % 16 == 0); then whichever is left
@@ -427,16 +427,20 @@ extern "C" int bn_r4_rows(const uint16_t *x, int64_t x_stride, const bn_r4 *w, i
   }
   if (M == 1) return N >= 8192 ? launch_rows<1, 2, false>(a, 1, s) : launch_rows<1, 1, false>(a, 1, s);
   if (M <= 8) {
-    int e = oct_rows(w, x, x_stride, M, N, K, y, y_stride, s);
-    if (e == -1) e = stream_rows(w, x, x_stride, M, N, K, y, y_stride, s);
-    if (e >= 0) return e;
-    // long rows, whose x does not fit beside the rings: two passes over the weights by half the rows
-    // each still beat the plain-load kernel (3840 x 15360: 81 us against 583 at four rows)
-    if (M > 2 && K % 16 == 0 && x_stride % 8 == 0) {
-      const int64_t half = M > 4 ? 4 : 2;
-      if (int e1 = bn_r4_rows(x, x_stride, w, half, N, K, y, y_stride, stream)) return e1;
-      return bn_r4_rows(x + half * x_stride, x_stride, w, M - half, N, K, y + half * y_stride, y_stride, stream);
+    auto pass = [&](int64_t m0, int64_t m) {
+      int e = oct_rows(w, x + m0 * x_stride, x_stride, m, N, K, y + m0 * y_stride, y_stride, s);
+      if (e == -1) e = stream_rows(w, x + m0 * x_stride, x_stride, m, N, K, y + m0 * y_stride, y_stride, s);
+      return e;
+    };
+    int e = pass(0, M);
+    // long rows, whose x does not fit beside the rings: passes over the weights by the most rows that
+    // do fit still beat one pass of the plain-load kernel (3840 x 15360: 81 us against 583 at four
+    // rows). Where no pass fits (more than 200 tiles, unaligned arrays) that one pass it is.
+    for (int64_t part = M > 4 ? 4 : 2; e == -1 && part >= 2 && part < M; part /= 2) {
+      e = pass(0, part);
+      if (e == BN_OK) return bn_r4_rows(x + part * x_stride, x_stride, w, M - part, N, K, y + part * y_stride, y_stride, stream);
     }
+    if (e >= 0) return e;
   }
   if (M == 2) return launch_rows<2, 2, false>(a, 1, s);
   if (M <= 4) return launch_rows<4, 2, false>(a, 1, s);

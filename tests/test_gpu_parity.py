@@ -707,6 +707,37 @@ def test_rows_of_many_row_matrices(N, K, M):
         assert np.array_equal(got[i], words(m(x[i]))), i
 
 
+def launches(f) -> int:
+    """Kernel launches of a call, counted as nodes of its CUDA graph."""
+    from cuda.bindings import runtime
+
+    f()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        f()
+    status, _, count = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
+    assert status == runtime.cudaError_t.cudaSuccess
+    return count
+
+
+@pytest.mark.parametrize("N,K,M,shift,passes", [(64, 25616, 3, 0, 1), (64, 25616, 8, 0, 1), (64, 28672, 4, 0, 1), (96, 1024, 4, 1, 1), (4100, 1024, 8, 3, 1), (64, 264, 8, 0, 1), (3840, 15360, 4, 0, 2), (3840, 15360, 8, 0, 4)])
+def test_passes_over_the_weights(N, K, M, shift, passes):
+    """Three to eight input rows are cut only where the parts fit a kernel with rings: rows of more
+    than 200 tiles, an x off its 16-byte boundary and K % 16 != 0 take one pass, long rows that
+    do not fit beside x one per two rows; the bits are the one-row kernel's."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    m = r4.R4Linear(r4.from_dense((torch.randn((N, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)))
+    x = torch.randn(M * K + shift, generator=g, device="cuda").to(torch.bfloat16)[shift:].view(M, K)
+    assert launches(lambda: ck.r4_rows(m._a, x, N, K)) == passes
+    got = words(ck.r4_rows(m._a, x, N, K))
+    for i in range(M):
+        assert np.array_equal(got[i], words(m(x[i].clone()))), i
+
+
 @pytest.mark.parametrize("E,n,D,tokens,topk", [(1, 704, 640, 2, 1), (8, 656, 1296, 5, 4), (33, 640, 704, 70, 3), (40, 704, 2816, 64, 8), (4, 1024, 4096, 90, 4), (3, 640, 16384, 9, 3)])
 def test_grouped_gather_shapes(E, n, D, tokens, topk):
     """Slots grouped by expert (groups of four and of eight, half-filled groups, empty experts, padding
