@@ -73,6 +73,9 @@ __device__ __forceinline__ bool mm_bar_wait(uint32_t bar, uint32_t parity) {
   atomicExch(&g_mma_error, 1);
   return false;
 }
+// The wait of a whole warp: every lane learns when some lane's gave up, so that the warp stays
+// together for what has to be executed by all of it (elect.sync, tcgen05.ld).
+__device__ __forceinline__ bool mm_bar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(BN_FULL, mm_bar_wait(bar, parity)); }
 // Whether the phase is over already; does not wait.
 __device__ __forceinline__ bool mm_bar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -85,7 +88,8 @@ __device__ __forceinline__ bool mm_bar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// True in one lane of the (converged) warp. Instructions that a single thread issues (MMAs, commits,
+// True in one lane of the warp, all of which has to get here: behind values that are the same in every
+// lane only. Instructions that a single thread issues (MMAs, commits,
 // bulk copies) take their operands from uniform registers; behind `lane == 0` the compiler has to
 // assume divergent values and wraps each of them in code that makes them uniform.
 __device__ __forceinline__ bool elect_one() {
@@ -198,7 +202,8 @@ __device__ __forceinline__ bool mma_issue_side(const CUtensorMap *x_map, const M
 // Warps 0..3: accumulators out of tensor memory (TMEM lane = weight row of the block), rounded to
 // BF16 and stored.
 __device__ __forceinline__ void mma_store_side(const MmaArgs &a, const MmaWindow &m, uint32_t tmem, uint32_t warp, uint32_t lane, int64_t row_base, int rows, bool ok, int mma_m = MMA_BM) {
-  if (ok) ok = mm_bar_wait(m.done, 0);
+  ok = __all_sync(BN_FULL, ok);  // (a decode warp's lanes wait on their own)
+  if (ok) ok = mm_bar_wait_warp(m.done, 0);
   tc_fence_after();
   const int r = mma_m == 64 ? (lane < 16 ? (int)(warp * 16 + lane) : MMA_BM) : (int)(warp * 32 + lane);  // M = 64: 16 rows in the lower half of each warp's lanes
   if (!ok) return;
@@ -585,10 +590,10 @@ __global__ void __launch_bounds__((MAXW + 2) * 32, 1) r4_mma_oct_kernel(const __
     // long as the tensor core needs for them), since the answer alone takes more than a hundred cycles
     bool have = false;
     for (int t = 0; t < T && ok; t++) {
-      if (!have) ok = mm_bar_wait(win.full + 8 * s, ph);
+      if (!have) ok = mm_bar_wait_warp(win.full + 8 * s, ph);
       const int ns = s + 1 == S ? 0 : s + 1;
       const uint32_t nph = ns ? ph : ph ^ 1u;
-      have = mm_bar_test(win.full + 8 * ns, nph);
+      have = __all_sync(BN_FULL, mm_bar_test(win.full + 8 * ns, nph));
       tc_fence_after();
       if (ok && elect_one()) {
         const uint64_t da = smem_desc(a_at + (uint32_t)s * a_stage), db = smem_desc(b_at + (uint32_t)s * b_stage);
@@ -619,7 +624,6 @@ __global__ void __launch_bounds__((MAXW + 2) * 32, 1) r4_mma_oct_kernel(const __
     }
     __syncwarp();
   }
-  ok = __all_sync(BN_FULL, ok);
   if (warp < 4) mma_store_side(a, win, tmem, warp, lane, row_base, rows, ok, pl.m);
   tc_fence_before();
   __syncthreads();
