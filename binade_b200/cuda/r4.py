@@ -219,6 +219,8 @@ class _R4:
             found[M] = left[0] if left else None
             if left:
                 self._cublas_split[M] = left[0]
+            else:  # nor may a split that an earlier call accepted stay
+                self._cublas_split.pop(M, None)
         return found
 
     def _rows(self, x: torch.Tensor) -> torch.Tensor:

@@ -306,3 +306,27 @@ def test_elected_lanes_follow_a_warp_vote():
     store = store[: store.index("tcgen05.ld")]
     assert "ok = __all_sync(BN_FULL, ok)" in store and not re.search(r"\bmm_bar_wait\(", store)
     assert re.search(r"bool mm_bar_wait_warp\([^)]*\) \{ return __all_sync\(BN_FULL, mm_bar_wait\(bar, parity\)\); \}", src)
+
+
+def test_mirror_cublas_forgets_a_rejected_split():
+    """A row count for which no split matches is run without one, whatever an earlier call found."""
+    import torch
+
+    from binade_b200.cuda import r4
+
+    class Product(r4._R4):  # stands in for the kernels: right for split 2 until it is `broken`
+        def __init__(self):
+            self.N, self.K, self.T, self.broken = 8, 256, 2, False
+            self.w = torch.randn((8, 256), generator=torch.Generator().manual_seed(0)).to(torch.bfloat16)
+
+        def dense(self):
+            return self.w
+
+        def mma_rows(self, x, split=None):
+            y = x @ self.w.T
+            return y if split == 2 and not self.broken else torch.zeros_like(y)
+
+    m = Product()
+    assert m.mirror_cublas(rows=(4, 16)) == {4: 2, 16: 2} and m._cublas_split == {4: 2, 16: 2}
+    m.broken = True
+    assert m.mirror_cublas(rows=(16,), seed=1) == {16: None} and m._cublas_split == {4: 2}
