@@ -7,14 +7,16 @@ namespace bn {
 namespace {
 
 constexpr int ROUTE_THREADS = 1024;
-constexpr int64_t ROUTE_EXPERTS = 48 * 1024;  // counters of this many experts fit shared memory
+constexpr int64_t ROUTE_EXPERTS = 48 * 1024;  // counters of this many experts fit shared memory; more are counted in seg
 
 // Slot g = choice g of the router, in token order: its expert (int32), input row g / k and its own
 // number; with seg, the slots grouped by expert besides: expert e's are order[seg[e] .. seg[e + 1])
 // (in no particular order: a slot's output does not depend on its neighbours). Ids outside 0 ..
 // E - 1 are in no group. One block.
 __global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const void *__restrict__ ids, int wide, int64_t G, int64_t k, int64_t E, uint32_t *__restrict__ ei, uint32_t *__restrict__ xi, uint32_t *__restrict__ iota, uint32_t *__restrict__ seg, uint32_t *__restrict__ order) {
-  extern __shared__ uint32_t counts[];  // [E], then running places
+  extern __shared__ uint32_t shared_counts[];
+  const bool in_seg = E > ROUTE_EXPERTS;
+  uint32_t *const counts = in_seg ? seg + 1 : shared_counts;  // [E], then running places: in the end, in seg, where the next expert's slots start
   __shared__ uint32_t warp_sum[32], carry;
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
   auto id = [&](int64_t g) { return wide ? (uint32_t)reinterpret_cast<const int64_t *>(ids)[g] : reinterpret_cast<const uint32_t *>(ids)[g]; };
@@ -45,12 +47,18 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const void *__rest
     __syncthreads();
     uint32_t before = carry;
     for (uint32_t w = 0; w < warp; w++) before += warp_sum[w];
-    if (e < E) seg[e] = counts[e] = before + upto - own;
+    if (e < E) {
+      counts[e] = before + upto - own;
+      if (!in_seg) seg[e] = counts[e];
+    }
     __syncthreads();
     if (threadIdx.x == ROUTE_THREADS - 1) carry = before + upto;
     __syncthreads();
   }
-  if (threadIdx.x == 0) seg[E] = carry;
+  if (threadIdx.x == 0) {
+    if (in_seg) seg[0] = 0;
+    else seg[E] = carry;
+  }
   for (int64_t g = threadIdx.x; g < G; g += ROUTE_THREADS) {
     const uint32_t e = id(g);
     if (e < E) order[atomicAdd(counts + e, 1u)] = (uint32_t)g;
@@ -79,9 +87,8 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const uint16_t *__restrict_
 
 extern "C" int bn_moe_route(const void *ids, int ids64, int64_t G, int64_t k, int64_t E, uint32_t *ei, uint32_t *xi, uint32_t *iota, uint32_t *seg, uint32_t *order, void *stream) {
   if (G < 0 || k < 1 || E < 0 || (G && !ids) || (seg && G && !order)) return bn::fail(BN_ERR_ARG, "bn_moe_route: null pointer or bad size");
-  if (seg && E > bn::ROUTE_EXPERTS) return bn::fail(BN_ERR_ARG, "bn_moe_route: too many experts to group");
   if (G == 0 && !seg) return BN_OK;
-  const size_t smem = seg ? (size_t)E * 4 : 0;
+  const size_t smem = seg && E <= bn::ROUTE_EXPERTS ? (size_t)E * 4 : 0;
   BN_CUDA(bn::allow_smem(bn::route_kernel, bn::ROUTE_EXPERTS * 4));
   bn::route_kernel<<<1, bn::ROUTE_THREADS, smem, (cudaStream_t)stream>>>(ids, ids64, G, k, E, ei, xi, iota, seg, order);
   return bn::launched("route_kernel");

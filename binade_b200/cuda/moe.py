@@ -54,7 +54,7 @@ class R4SwitchGLU(nn.Module):
         return self._run(x, xi, ei, rows, ck.group_slots(ei, self.E) if self._grouped(ei.numel()) else None, max_per_expert or x.shape[0])
 
     def _grouped(self, G: int) -> bool:
-        return G >= self.GROUP_MIN_SLOTS * self.E and self.E <= 48 * 1024
+        return G >= self.GROUP_MIN_SLOTS * self.E
 
     def _run(self, x, xi, ei, rows, groups, cap: int) -> torch.Tensor:
         n = self.n

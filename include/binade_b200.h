@@ -271,7 +271,7 @@ int bn_r4_gather_grouped(const uint16_t *x, const bn_r4 *w, const uint32_t *xi, 
 /* The router's choices as slots: ids [G] (int64 if ids64, else int32), k a token, in token order ->
  * ei [G] expert, xi [G] = g / k, iota [G] = g; with seg [E+1] and order [G] the slots grouped by expert:
  * expert e's are order[seg[e]] .. order[seg[e+1] - 1], in any order; ids outside 0 .. E-1 are in no
- * group. Any output may be NULL (order goes with seg). E <= 49152 with seg. */
+ * group. Any output may be NULL (order goes with seg). */
 int bn_moe_route(const void *ids, int ids64, int64_t G, int64_t k, int64_t E, uint32_t *ei, uint32_t *xi,
                  uint32_t *iota, uint32_t *seg, uint32_t *order, void *stream);
 

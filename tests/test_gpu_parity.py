@@ -767,6 +767,36 @@ def test_grouped_gather_shapes(E, n, D, tokens, topk):
         assert np.array_equal(words(a[real]), words(b[real]))
 
 
+@pytest.mark.parametrize("E,G", [(49152, 3000), (49153, 3000), (65000, 1), (200000, 70000)])
+def test_grouping_of_many_experts(E, G):
+    """More experts than shared memory has counters for; ids outside the experts are in no group."""
+    from binade_b200.cuda import kernels as ck
+
+    rng = np.random.default_rng(E)
+    ids = rng.integers(-3, E + 3, G).astype(np.int32)
+    ids[: G // 2] = ids[G // 2 : G // 2 + G // 2] // 1000
+    seg, order = (t.cpu().numpy() for t in ck.group_slots(dev(ids), E))
+    real = ids[(ids >= 0) & (ids < E)]
+    assert np.array_equal(seg, np.concatenate([[0], np.cumsum(np.bincount(real, minlength=E))]))
+    for e in np.unique(real):
+        assert np.array_equal(np.sort(order[seg[e] : seg[e + 1]]), np.flatnonzero(ids == e)), e
+
+
+def test_grouped_gather_of_many_experts():
+    """A grouped gather over more experts than shared memory has counters for."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+
+    E, n, K, G = 50000, 2, 640, 40
+    g = torch.Generator(device="cuda").manual_seed(3)
+    m = r4.R4Linear(r4.from_dense((torch.randn((E * n, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)))
+    x = torch.randn((G, K), generator=g, device="cuda").to(torch.bfloat16)
+    ei = torch.randint(0, E, (G,), generator=g, device="cuda").to(torch.int32)
+    ei[1::2] = ei[::2]
+    xi = torch.arange(G, dtype=torch.int32, device="cuda")
+    assert np.array_equal(words(ck.r4_gather_grouped(m._a, x, xi, ei, E, 2, n, n, 0, K)), words(m._gather(x, xi, ei, n, n)))
+
+
 @pytest.mark.parametrize("n", [1, 2, 511, 513, 704 * 8])
 def test_swiglu_bits(n):
     """The activation's kernel against torch's fp32 silu and product, bit for bit, infinities and NaN
