@@ -11,6 +11,7 @@ struct RiceArgs {
   const uint8_t *meta;
   const uint32_t *bits;
   uint64_t nwords;
+  uint32_t shift;  // the stream's first word is bits[shift]: `bits` rounded down to 16 bytes (rice_tiles.cu)
   const uint32_t *roff;
   const uint8_t *table;
   const uint8_t *raw;
@@ -49,7 +50,7 @@ __device__ __forceinline__ uint32_t low_mask(int n) {
 // Decode in two kernels, one thread per tile (rice_tiles.cu); -1 when the arrays are outside their
 // coverage. rice_tiles_r4 fills what rice_kernel<RICE_R4> fills, rice_tiles_unpack what
 // rice_kernel<RICE_UNPACK> fills.
-int rice_tiles_r4(const RiceArgs &a, cudaStream_t s);
-int rice_tiles_unpack(const RiceArgs &a, cudaStream_t s);
+int rice_tiles_r4(RiceArgs a, cudaStream_t s);
+int rice_tiles_unpack(RiceArgs a, cudaStream_t s);
 
 }  // namespace bn

@@ -7,8 +7,8 @@
 //   unary planes  j = 0 .. qmax-1: one bit per weight still alive (q >= j), set iff q > j
 // The bit offset of a lane inside a plane is the number of alive weights before it: a warp
 // prefix sum over per-lane alive counts, done with three ballots. These kernels take what the faster
-// decoder with a thread per tile (rice_tiles.cu) does not: ranks, K % 4 != 0, unaligned arrays, and
-// format 1.
+// decoder with a thread per tile (rice_tiles.cu) does not: ranks, K % 4 != 0, raw bytes and BF16
+// rows off a 16-byte boundary, and format 1.
 #include <atomic>
 
 #include "rice.cuh"
@@ -333,7 +333,7 @@ static int rice_grid(int64_t R) {
   return (int)(blocks < cap ? blocks : cap);
 }
 
-// A thread per tile where the arrays allow it (16-byte aligned stream), else a warp per row.
+// A thread per tile where the arrays allow it (K % 4 == 0, codes on 8 bytes), else a warp per row.
 static int launch_rice_r4(const RiceArgs &a, cudaStream_t s) {
   const int e = rice_tiles_r4(a, s);
   if (e != -1) return e;
@@ -341,7 +341,7 @@ static int launch_rice_r4(const RiceArgs &a, cudaStream_t s) {
   return launched("rice_kernel<r4>");
 }
 
-// BF16 rows alike (K % 4 == 0, 16-byte aligned arrays).
+// BF16 rows alike (K % 4 == 0, raw bytes and rows on 16 bytes).
 static int launch_rice_unpack(const RiceArgs &a, cudaStream_t s) {
   const int e = rice_tiles_unpack(a, s);
   if (e != -1) return e;

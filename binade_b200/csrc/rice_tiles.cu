@@ -29,8 +29,10 @@ constexpr uint32_t SC_BLOCK = 128;                   // words of a ring block
 constexpr uint32_t SC_RING = 2 * SC_BLOCK;           // words of a row's ring
 constexpr uint32_t SC_STRIDE = SC_RING + 12;         // the ring's first 12 words again at its end: a read of up to 12 words never wraps
 
-// Words outside [0, nwords) read as zero.
+// Words from nwords on read as zero.
 __device__ __forceinline__ uint32_t word_at(const uint32_t *__restrict__ bits, uint64_t nwords, uint64_t i) { return i < nwords ? __ldg(bits + i) : 0u; }
+// First word of a row in `bits` (an offset past every stream stays one).
+__device__ __forceinline__ uint32_t row_word(const RiceArgs &a, int64_t row) { return min(a.roff[row], 0xFFFFFFFFu - a.shift) + a.shift; }
 // (hi:lo) >> n, n <= 32
 __device__ __forceinline__ void shift_out(uint32_t &lo, uint32_t &hi, uint32_t n) {
   lo = __funnelshift_rc(lo, hi, n);
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(32) rice_scan_kernel(RiceArgs a, uint8_t *slot
     srow = live ? (int64_t)a.ids[row] : 0;
     if (srow >= a.rows) live = false, srow = 0;  // an id outside the table: the decode writes zeros
   }
-  const uint32_t w0 = live ? a.roff[srow] : 0u;
+  const uint32_t w0 = live ? row_word(a, srow) : 0u;
   const uint32_t first = w0 & ~3u;  // the ring starts at a 16-byte boundary of the stream
   const uint32_t avail = (uint64_t)first < a.nwords ? (uint32_t)min(a.nwords - first, (uint64_t)0xFFFFFFFFu) : 0u;
   const uint32_t off = (w0 & 3u) * 32u;
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(32) rice_scan_kernel(RiceArgs a, uint8_t *slot
     usable = req;
     if (!__any_sync(BN_FULL, t < T)) break;
   }
-  const uint32_t rend = w0 + ((cur - off + 31u) >> 5);
+  const uint32_t rend = w0 - a.shift + ((cur - off + 31u) >> 5);
   if (MODE == RICE_R4) {
     // escape scratch for the most escapes the rows' meta bytes allow, claimed once per warp
     uint32_t upto = bound;
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(32) rice_scan_kernel(RiceArgs a, uint8_t *slot
     claim = __shfl_sync(BN_FULL, claim, 31);
     if (!live || part) return;
     a.tmp_off[row] = claim + upto - bound;
-    const uint64_t w_end = row + 1 < a.R ? (uint64_t)a.roff[row + 1] : a.nwords;
+    const uint64_t w_end = row + 1 < a.R ? (uint64_t)a.roff[row + 1] : a.nwords - a.shift;
     if ((uint64_t)rend != w_end) atomicMax(a.counters + 1, (uint32_t)(a.R - row));
   } else if (live && part == 0 && a.rend) {
     a.rend[row] = rend;
@@ -268,6 +270,7 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the tiles' first bits
 
   const int T = a.T;
+  const bool quads = !(reinterpret_cast<uintptr_t>(a.codes) & 15);  // (8-byte aligned else)
   const int64_t K = a.K, tasks = (a.R + rows_per_task - 1) / rows_per_task;
   uint32_t escapes = 0;  // of the rows whose count this lane stores
   for (int64_t task = (int64_t)warp * gridDim.x + blockIdx.x; task < tasks; task += (int64_t)gridDim.x * TI_WARPS) {
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
       const uint32_t m = a.meta[srow * T + t], k = m & 3u, qmax = m >> 2;
       const uint32_t n = (uint32_t)min((int64_t)BN_TILE, K - (int64_t)t * BN_TILE);
       const uint32_t *const slot = reinterpret_cast<const uint32_t *>(slots + (row + 1) * row_bytes) - T;
-      const uint32_t w0 = a.roff[srow], begin = slot[t], end = t + 1 < T ? slot[t + 1] : begin + n * (k + qmax);
+      const uint32_t w0 = row_word(a, srow), begin = slot[t], end = t + 1 < T ? slot[t + 1] : begin + n * (k + qmax);
       const uint32_t first_word = w0 + (begin >> 5), last_word = w0 + (end >> 5);
       // the raw bytes are only needed once the tiles are decoded: on their way to L2 meanwhile
       if (MODE == RICE_UNPACK && mine) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.raw + srow * K + (int64_t)t * BN_TILE));
@@ -434,7 +437,11 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
         if (MODE == RICE_R4) {
           const int64_t tile0 = row0 * T + t0 + from;  // the chunk's tiles are consecutive in memory
           uint4 *const dst = reinterpret_cast<uint4 *>(a.codes + tile0 * 32);
-          for (int i = (int)lane; i < (to - from) * 4; i += 32) dst[i] = *reinterpret_cast<const uint4 *>(sc + (from + (i >> 2)) * TI_TILE + (i & 3) * 4);
+          for (int i = (int)lane; i < (to - from) * 4; i += 32) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(sc + (from + (i >> 2)) * TI_TILE + (i & 3) * 4);
+            if (quads) dst[i] = v;
+            else reinterpret_cast<uint2 *>(dst + i)[0] = make_uint2(v.x, v.y), reinterpret_cast<uint2 *>(dst + i)[1] = make_uint2(v.z, v.w);
+          }
           if (active) a.flags[row0 * T + t0 + lane] = count != 0;
           if (!active) count = 0;
           if (__any_sync(BN_FULL, count != 0)) {
@@ -557,19 +564,26 @@ int launch_tiles(const RiceArgs &a, uint8_t *slots, int64_t row_bytes, cudaStrea
   return launched("rice_tiles_kernel");
 }
 
-bool tiles_cover(const RiceArgs &a) {
-  return a.K % 4 == 0 && !(reinterpret_cast<uintptr_t>(a.bits) & 15) && a.T <= (1 << 18) && a.R <= (1ll << 31);
+// Streams may start on any word (a shard uploaded whole, with pointers into it): `bits` is rounded
+// down to the 16 bytes that the kernels read at a time, which stay inside the caller's allocation.
+// false: outside the kernels' coverage.
+bool tiles_cover(RiceArgs &a) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a.bits);
+  a.shift = (uint32_t)(at & 15) / 4;
+  if (a.K % 4 || at & 3 || a.T > (1 << 18) || a.R > (1ll << 31) || (a.shift && a.nwords > 0xFFFFFFF0u)) return false;
+  a.bits -= a.shift, a.nwords += a.shift;
+  return true;
 }
 
 }  // namespace
 
-int rice_tiles_r4(const RiceArgs &a, cudaStream_t s) {
-  if (!tiles_cover(a) || (reinterpret_cast<uintptr_t>(a.codes) & 15)) return -1;
+int rice_tiles_r4(RiceArgs a, cudaStream_t s) {
+  if ((reinterpret_cast<uintptr_t>(a.codes) & 7) || !tiles_cover(a)) return -1;
   return launch_tiles<RICE_R4>(a, reinterpret_cast<uint8_t *>(a.codes), (int64_t)a.T * 64, s);
 }
 
-int rice_tiles_unpack(const RiceArgs &a, cudaStream_t s) {
-  if (!tiles_cover(a) || ((reinterpret_cast<uintptr_t>(a.raw) | reinterpret_cast<uintptr_t>(a.out)) & 15)) return -1;
+int rice_tiles_unpack(RiceArgs a, cudaStream_t s) {
+  if (((reinterpret_cast<uintptr_t>(a.raw) | reinterpret_cast<uintptr_t>(a.out)) & 15) || !tiles_cover(a)) return -1;
   return launch_tiles<RICE_UNPACK>(a, reinterpret_cast<uint8_t *>(a.out), a.K * 2, s);
 }
 

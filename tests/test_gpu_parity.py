@@ -34,6 +34,20 @@ def weights(rng, shape, scale=0.02, escapes=True):
     return u
 
 
+def launches(f) -> int:
+    """Kernel launches of a call, counted as nodes of its CUDA graph."""
+    from cuda.bindings import runtime
+
+    f()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        f()
+    status, _, count = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
+    assert status == runtime.cudaError_t.cudaSuccess
+    return count
+
+
 def words(t: torch.Tensor) -> np.ndarray:
     return t.contiguous().view(torch.int16).cpu().numpy().view(np.uint16)
 
@@ -302,6 +316,42 @@ def test_thread_per_tile_codec(N, K, kind):
     ids = np.array([N - 1, 0, N, N // 2, 0], np.int32)
     rows = words(ck.rice_lookup(d["meta"].reshape(-1), d["bits"], d["roff"], d["table"], d["raw"], N, K, ck.to_device(ids)))
     assert np.array_equal(rows, np.where((ids < N)[:, None], u[np.minimum(ids, N - 1)], np.uint16(0)))
+
+
+@pytest.mark.parametrize("N,K,kind", [(9, 4100, "normal"), (700, 2048, "uniform"), (20001, 260, "normal"), (40000, 128, "normal")])
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_streams_on_any_word(N, K, kind, shift):
+    """Streams that start off a 16-byte boundary, behind other words, and codes on 8 bytes: the arrays and
+    rows of an aligned stream, by as many launches."""
+    from binade_b200.cuda import kernels as ck
+
+    rng = np.random.default_rng(N + shift)
+    u = weights(rng, (N, K)) if kind == "normal" else rng.integers(0, 1 << 16, (N, K)).astype(np.uint16)
+    p, T = packed_arrays(u), -(-K // 128)
+    d = {k: ck.to_device(p[k]).reshape(-1) for k in ("raw", "table", "meta", "bits", "roff")}
+    words_in = d["bits"].numel()
+    off = torch.full((words_in + 8,), -1, dtype=torch.int32, device="cuda")[shift : shift + words_in]
+    off.copy_(d["bits"])
+    assert d["bits"].data_ptr() % 16 == 0 and off.data_ptr() % 16 == 4 * shift
+    results, counts = [], []
+    for bits, lead in ((d["bits"], 0), (off, 4)):
+        codes = torch.empty(N * T * 32 + lead, dtype=torch.int16, device="cuda")[lead:]
+        flags, esc = torch.empty(N * T, dtype=torch.uint8, device="cuda"), torch.zeros(N * K, dtype=torch.uint8, device="cuda")
+        cnt, at, ctr = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (N, N, 8))
+        call = lambda: ck._call("bn_rice_to_r4", ck._p(d["meta"]), ck._p(bits), words_in, ck._p(d["roff"]), ck._p(d["table"]), N, K, ck._p(codes), ck._p(flags), ck._p(cnt), ck._p(esc), N * K, ck._p(at), ck._p(ctr))  # noqa: E731
+        read = lambda: ck.rice_unpack(d["meta"], bits, d["roff"], d["table"], d["raw"], N, K)  # noqa: E731
+        counts.append((launches(call), launches(read)))
+        call()
+        assert ctr[1] == 0
+        out = torch.empty(int(ctr[2]) + 1, dtype=torch.uint8, device="cuda")
+        rows = torch.empty_like(cnt)
+        ck._call("bn_r4_finish", ck._p(cnt), ck._p(esc), ck._p(at), N, ck._p(rows), ck._p(out), out.numel())
+        w, rend = read()
+        assert np.array_equal(words(w), u)
+        results.append((codes, flags, cnt, out, rows, rend))
+    assert counts[0] == counts[1]
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
 
 
 def test_transcode_all_escapes_grows_scratch():
@@ -705,20 +755,6 @@ def test_rows_of_many_row_matrices(N, K, M):
     got = words(m.fused_rows(x))
     for i in range(M):
         assert np.array_equal(got[i], words(m(x[i]))), i
-
-
-def launches(f) -> int:
-    """Kernel launches of a call, counted as nodes of its CUDA graph."""
-    from cuda.bindings import runtime
-
-    f()
-    torch.cuda.synchronize()
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph):
-        f()
-    status, _, count = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
-    assert status == runtime.cudaError_t.cudaSuccess
-    return count
 
 
 @pytest.mark.parametrize("N,K,M,shift,passes", [(64, 25616, 3, 0, 1), (64, 25616, 8, 0, 1), (64, 28672, 4, 0, 1), (96, 1024, 4, 1, 1), (4100, 1024, 8, 3, 1), (64, 264, 8, 0, 1), (3840, 15360, 4, 0, 2), (3840, 15360, 8, 0, 4)])
