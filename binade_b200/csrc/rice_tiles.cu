@@ -39,18 +39,29 @@ __device__ __forceinline__ void shift_out(uint32_t &lo, uint32_t &hi, uint32_t n
   asm("shr.b32 %0, %0, %1;" : "+r"(hi) : "r"(n));
 }
 
-// Bit after the tile that starts at bit `cur` of a row whose first word is bits[w0], read from
-// global memory: tiles too long for the ring.
-__device__ __noinline__ uint32_t scan_long_tile(const uint32_t *__restrict__ bits, uint64_t nwords, uint64_t w0, uint32_t cur, uint32_t n, uint32_t k, uint32_t qmax) {
-  uint32_t pos = cur + n * k, len = n;
-  for (uint32_t j = 0; j < qmax && len; j++) {
-    uint32_t ones = 0;
-    for (uint32_t done = 0; done < len; done += 32) {
-      const uint32_t p = pos + done;
-      const uint64_t w = w0 + (p >> 5);
-      ones += __popc(__funnelshift_r(word_at(bits, nwords, w), word_at(bits, nwords, w + 1), p & 31u) & low_mask((int)(len - done)));
-    }
+// Bit after the tile that starts at bit `cur` of the row's ring space, for tiles that might not fit the
+// ring: words before `limit` come from there, the others from global memory (`row` is where the
+// ring space starts). The four lanes of a row count 32 bits of a plane each.
+__device__ __noinline__ uint32_t scan_long_tile(const uint32_t *__restrict__ bits, uint64_t nwords, uint64_t row, uint32_t ring, uint32_t limit, uint32_t cur, uint32_t n, uint32_t k, uint32_t qmax) {
+  const uint32_t lane = lane_id(), mask = 15u << (lane & 28u);
+  auto word = [&](uint32_t w) { return w < limit ? lds_u32(ring + 4u * (w & (SC_RING - 1u))) : word_at(bits, nwords, row + w); };
+  uint32_t pos = cur + n * k, len = n, j = 0;
+  for (; j < qmax && len > 32u; j++) {
+    const uint32_t at = pos + 32u * (lane & 3u), w = at >> 5;
+    uint32_t ones = __popc(__funnelshift_r(word(w), word(w + 1u), at & 31u) & low_mask((int)(len - 32u * (lane & 3u))));
+    ones += __shfl_xor_sync(mask, ones, 1);
+    ones += __shfl_xor_sync(mask, ones, 2);
     pos += len, len = ones;
+  }
+  uint32_t lo = 0, hi = 0, room = 0;  // a window of the bits from pos on
+  for (; j < qmax && len; j++) {
+    if (len > room) {
+      const uint32_t w = pos >> 5, v = word(w + 1u);
+      lo = __funnelshift_r(word(w), v, pos & 31u), hi = __funnelshift_r(v, word(w + 2u), pos & 31u), room = 64;
+    }
+    const uint32_t ones = __popc(lo & low_mask((int)len));
+    shift_out(lo, hi, len);
+    pos += len, room -= len, len = ones;
   }
   return pos;
 }
@@ -111,13 +122,15 @@ __global__ void __launch_bounds__(32) rice_scan_kernel(RiceArgs a, uint8_t *slot
       const uint32_t n = (uint32_t)min((int64_t)BN_TILE, a.K - (int64_t)t * BN_TILE);
       const uint32_t most = n * (k + qmax);
       const bool is_long = most > SC_BLOCK * 32u;
-      const bool go = t < T && (is_long || cur + most <= usable * (SC_BLOCK * 32u));
+      // (a long tile starts with both blocks of the ring at hand)
+      const uint32_t need = min(most, 2u * SC_BLOCK * 32u - (cur & (SC_BLOCK * 32u - 1u)));
+      const bool go = t < T && cur + need <= usable * (SC_BLOCK * 32u);
       if (!__any_sync(BN_FULL, go)) break;
       if (go) {
         if (part == 0) slot[t] = cur - off;
         if (t + 1 < T) m_next = meta[t + 1];
         if (MODE == RICE_R4 && part == 0 && ((qmax << k) | ((1u << k) - 1u)) >= 15u) bound += n;  // only such a tile can hold a rank >= 15
-        if (is_long) cur = scan_long_tile(a.bits, a.nwords, first, cur, n, k, qmax);
+        if (is_long) cur = scan_long_tile(a.bits, a.nwords, first, smem_addr(ring), usable * SC_BLOCK, cur, n, k, qmax);
         t++;
       }
       const uint32_t planes = go && !is_long ? qmax : 0u;
@@ -192,20 +205,6 @@ __device__ __forceinline__ uint32_t window(const uint32_t *sw, uint32_t pos) {
   const uint32_t *p = sw + (pos >> 5);
   return __funnelshift_r(p[0], p[1], pos & 31u);
 }
-__device__ uint32_t count_ones(const uint32_t *sw, uint32_t pos, uint32_t len) {
-  uint32_t c = 0;
-  for (uint32_t done = 0; done < len; done += 32) c += __popc(window(sw, pos + done) & low_mask((int)(len - done)));
-  return c;
-}
-// Quotient of weight `i` of a tile whose first plane starts at bit `pos`.
-__device__ __noinline__ uint32_t quotient_of(const uint32_t *sw, uint32_t pos, uint32_t n, uint32_t qmax, uint32_t i) {
-  uint32_t len = n, q = 0;
-  while (q < qmax && (window(sw, pos + i) & 1u)) {
-    const uint32_t before = count_ones(sw, pos, i), ones = before + count_ones(sw, pos + i, len - i);
-    pos += len, len = ones, i = before, q++;
-  }
-  return q;
-}
 // Bits 2m of x packed together (16 of them).
 __device__ __forceinline__ uint32_t pack2(uint32_t x) {
   x &= 0x55555555u;
@@ -213,14 +212,6 @@ __device__ __forceinline__ uint32_t pack2(uint32_t x) {
   x = (x | (x >> 2)) & 0x0F0F0F0Fu;
   x = (x | (x >> 4)) & 0x00FF00FFu;
   return (x | (x >> 8)) & 0xFFFFu;
-}
-// Bits 3m of x packed together (10 of them).
-__device__ __forceinline__ uint32_t pack3(uint32_t x) {
-  x &= 0x09249249u;
-  x = (x | (x >> 2)) & 0x030C30C3u;
-  x = (x | (x >> 4)) & 0x0300F00Fu;
-  x = (x | (x >> 8)) & 0x030000FFu;
-  return (x | (x >> 16)) & 0x3FFu;
 }
 // Bit planes r0..r3 of 32 nibbles -> the nibbles, eight a word, in order.
 __device__ __forceinline__ uint4 nibbles(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
@@ -314,10 +305,12 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
         __syncwarp();
         const bool active = (int)lane >= from && (int)lane < to;
         if (active) low_at = (first_word - base) * 32u + (begin & 31u), planes_at = low_at + n * k;
+        const uint32_t shared_tiles = __ballot_sync(BN_FULL, active && k == 3);  // the warp decodes each together
+        const bool own = active && k < 3;
         uint32_t alive[4], q0[4], q1[4], q2[4], q3[4], sat[4];
         const uint32_t q_top = 15u >> k;  // quotients above it mean rank >= 15
-        uint32_t pos = active ? planes_at : 0u;
-        const bool coded = active && qmax > 0;
+        uint32_t pos = own ? planes_at : 0u;
+        const bool coded = own && qmax > 0;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
           alive[i] = coded ? window(sw, pos + 32 * i) & low_mask((int)n - 32 * i) : 0u;  // plane 0
@@ -378,7 +371,7 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
           }
         }
         // the low bits as bit planes under the quotients'
-        if (active) {
+        if (own) {
 #pragma unroll
           for (int i = 0; i < 4; i++) {
             const uint32_t valid = low_mask((int)n - 32 * i);
@@ -387,17 +380,10 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
               r3 = r2, r2 = r1, r1 = r0;
               if (k == 1) {
                 r0 = window(sw, low_at + 32 * i) & valid;
-              } else if (k == 2) {
+              } else {
                 r3 = r2, r2 = r1;
                 const uint32_t x = valid ? window(sw, low_at + 64 * i) : 0u, y = valid & 0xFFFF0000u ? window(sw, low_at + 64 * i + 32) : 0u;
                 r0 = (pack2(x) | (pack2(y) << 16)) & valid, r1 = (pack2(x >> 1) | (pack2(y >> 1) << 16)) & valid;
-              } else {
-                r3 = r1, r0 = r1 = r2 = 0u;
-                for (int c = 0; c < 4; c++) {
-                  const uint32_t x = (valid >> (10 * c)) ? window(sw, low_at + 96 * i + 30 * c) : 0u;
-                  r0 |= pack3(x) << (10 * c), r1 |= pack3(x >> 1) << (10 * c), r2 |= pack3(x >> 2) << (10 * c);
-                }
-                r0 &= valid, r1 &= valid, r2 &= valid;
               }
             }
             r0 |= sat[i], r1 |= sat[i], r2 |= sat[i], r3 |= sat[i];
@@ -420,21 +406,88 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
           }
           count = __popc(hits[0]) + __popc(hits[1]) + __popc(hits[2]) + __popc(hits[3]);
         }
-        // exponents of the escaped weights (rank >= 15), in order
+        // exponents of the escaped weights (rank >= 15) with their place among the tile's: of the few
+        // by their counts; the others' quotients are where they die in one more walk over the
+        // planes, which such a tile alone takes
         auto each_escape = [&](auto &&put) {
-          uint32_t c = 0;  // of the few: those before this word
+          uint32_t c = 0, hits_before[4], left[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) hits_before[i] = c, c += __popc(hits[i]), left[i] = hits[i] & ~alive[i];
+          auto place = [&](int i, uint32_t bit, uint32_t q) {
+            const uint32_t at = 32u * i + (uint32_t)__ffs((int)bit) - 1u;
+            put(at, (uint32_t)tbl[((q << k) | (k ? window(sw, low_at + at * k) & ((1u << k) - 1u) : 0u)) & 0xFFu], hits_before[i] + __popc(hits[i] & (bit - 1u)));
+          };
+          c = 0;  // of the few: those before this word
 #pragma unroll
           for (int i = 0; i < 4; i++) {
-            for (uint32_t h = hits[i]; h; h &= h - 1u) {
-              const uint32_t bit = h & (0u - h), at = 32u * i + (uint32_t)__ffs((int)h) - 1u;
-              const uint32_t q = alive[i] & bit ? j + (__byte_perm(more0, more1, 0x4440u | (c + __popc(alive[i] & (bit - 1u)))) & 0xFFu) : quotient_of(sw, planes_at, n, qmax, at);
-              put(at, (uint32_t)tbl[((q << k) | (k ? window(sw, low_at + at * k) & ((1u << k) - 1u) : 0u)) & 0xFFu]);
+            for (uint32_t h = hits[i] & alive[i]; h; h &= h - 1u) {
+              const uint32_t bit = h & (0u - h);
+              place(i, bit, j + (__byte_perm(more0, more1, 0x4440u | (c + __popc(alive[i] & (bit - 1u)))) & 0xFFu));
             }
             c += __popc(alive[i]);
+          }
+          uint32_t live[4], at = planes_at;
+#pragma unroll
+          for (int i = 0; i < 4; i++) live[i] = low_mask((int)n - 32 * i);
+          for (uint32_t q = 0; left[0] | left[1] | left[2] | left[3]; q++) {  // (alive after the last plane: q = qmax)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              uint32_t bits = window(sw, at), next = 0;
+              at += __popc(live[i]);
+#pragma unroll
+              for (int b = 0; b < 4; b++) {
+                next |= (uint32_t)deposit[__byte_perm(bits, live[i], 0x40 + 0x10 * b) & 0xFFFFu] << (8 * b);
+                bits >>= __popc(live[i] & (0xFFu << (8 * b)));
+              }
+              if (q >= qmax) next = 0;
+              for (uint32_t h = left[i] & ~next; h; h &= h - 1u) place(i, h & (0u - h), q);
+              live[i] = next, left[i] &= next;
+            }
+          }
+        };
+        // tiles with k = 3, one after the other: four weights a lane, their ranks in the bytes of a word
+        auto each_shared = [&](auto &&take) {
+          for (uint32_t rest = shared_tiles; rest; rest &= rest - 1u) {
+            const int u = __ffs((int)rest) - 1;
+            const uint32_t un = __shfl_sync(BN_FULL, n, u), planes = __shfl_sync(BN_FULL, qmax, u), low = __shfl_sync(BN_FULL, low_at, u);
+            const uint32_t nv = (uint32_t)max(0, min(4, (int)un - 4 * (int)lane));
+            uint32_t four = (1u << nv) - 1u, q = 0, at = low + 3u * un;
+            for (uint32_t plane = 0; plane < planes; plane++) {
+              const uint32_t c = __popc(four);
+              uint32_t before, all;
+              warp_scan_small(c, lanemask_lt(), before, all);
+              if (!all) break;
+              four = small[four | ((window(sw, at + before) & low_mask((int)c)) << 4)];  // the survivors
+              q += (four * 0x00204081u) & 0x01010101u;
+              at += all;
+            }
+            const uint32_t x = nv ? window(sw, low + 12u * lane) : 0u;
+            const uint32_t lows = (x & 7u) | ((x << 5) & 0x700u) | ((x << 10) & 0x70000u) | ((x << 15) & 0x7000000u);
+            take(u, nv, (((q & 0x1F1F1F1Fu) << 3) | lows) & low_mask((int)(8u * nv)));
           }
         };
         __syncwarp();
         if (MODE == RICE_R4) {
+          const uint64_t esc_at = (uint64_t)a.tmp_off[row] + (rows_per_task > 1 ? __shfl_sync(BN_FULL, row_escapes, mine ? sub * T : 0) : row_escapes);  // of this lane's row, the chunk's earlier ones included
+          each_shared([&](int u, uint32_t, uint32_t ranks) {
+            const uint32_t over = (((ranks & 0x7F7F7F7Fu) + 0x71717171u) | ranks) & 0x80808080u;  // bit 7 of the bytes from 15 on
+            uint32_t c = (ranks | ((over >> 7) * 15u)) & 0x0F0F0F0Fu;
+            c = (c | (c >> 4)) & 0x00FF00FFu;
+            reinterpret_cast<uint16_t *>(sc + u * TI_TILE)[lane] = (uint16_t)(c | (c >> 8));
+            const int usub = __shfl_sync(BN_FULL, sub, u);
+            const uint32_t earlier = __reduce_add_sync(BN_FULL, (int)lane < u && sub == usub && active ? count : 0u);
+            uint32_t before, all;
+            warp_scan_small(__popc(over), lanemask_lt(), before, all);
+            uint64_t p = __shfl_sync(BN_FULL, esc_at, u) + earlier + before;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+              if ((over >> (8 * i + 7)) & 1u) {
+                if (p < a.esc_cap) a.esc_tmp[p] = tbl[(ranks >> (8 * i)) & 0xFFu];
+                p++;
+              }
+            if ((int)lane == u) count = all;
+          });
+          __syncwarp();
           const int64_t tile0 = row0 * T + t0 + from;  // the chunk's tiles are consecutive in memory
           uint4 *const dst = reinterpret_cast<uint4 *>(a.codes + tile0 * 32);
           for (int i = (int)lane; i < (to - from) * 4; i += 32) {
@@ -454,11 +507,9 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
             const uint32_t total = __shfl_sync(BN_FULL, upto, 31);
             // several rows a task: positions count from the row's first tile
             const uint32_t before = __shfl_sync(BN_FULL, upto - count, rows_per_task > 1 ? max(sub * T, from) & 31 : 0);
-            const uint32_t carried = rows_per_task > 1 ? __shfl_sync(BN_FULL, row_escapes, mine ? sub * T : 0) : row_escapes;
-            uint64_t p = (uint64_t)a.tmp_off[row] + carried + (upto - count) - (rows_per_task > 1 ? before : 0u);
-            if (count) each_escape([&](uint32_t, uint32_t e) {
-              if (p < a.esc_cap) a.esc_tmp[p] = (uint8_t)e;
-              p++;
+            const uint64_t p = esc_at + (upto - count) - (rows_per_task > 1 ? before : 0u);
+            if (own && count) each_escape([&](uint32_t, uint32_t e, uint32_t index) {
+              if (p + index < a.esc_cap) a.esc_tmp[p + index] = (uint8_t)e;
             });
             if (rows_per_task == 1) {
               row_escapes += total;
@@ -479,7 +530,7 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
           auto fetch = [&](int u0) {
             const int u = u0 + (int)(lane >> 3);
             const int us = __shfl_sync(BN_FULL, sub, u & 31), ut = __shfl_sync(BN_FULL, t, u & 31);
-            Piece x{row0 + us, u < to ? (int64_t)ut * BN_TILE + (lane & 7u) * 16 : K, {0, 0, 0, 0}};
+            Piece x{row0 + us, u < to && !((shared_tiles >> u) & 1u) ? (int64_t)ut * BN_TILE + (lane & 7u) * 16 : K, {0, 0, 0, 0}};
             const uint8_t *const raw = a.raw + (a.ids ? srow : x.row) * K + x.col;
             if (wide && x.col < K) {
               const uint4 v = __ldg(reinterpret_cast<const uint4 *>(raw));
@@ -515,10 +566,17 @@ __global__ void __launch_bounds__(TI_WARPS * 32, 1) rice_tiles_kernel(RiceArgs a
             }
           }
           __syncwarp();  // the escaped weights' words are written over what went out above
-          if (active && count) each_escape([&](uint32_t i, uint32_t e) {
+          if (own && count) each_escape([&](uint32_t i, uint32_t e, uint32_t) {
             const int64_t col = (int64_t)t * BN_TILE + i;
             const uint32_t b = a.raw[srow * K + col];
             a.out[row * K + col] = (uint16_t)(((b & 0x80u) << 8) | (e << 7) | (b & 0x7Fu));
+          });
+          each_shared([&](int u, uint32_t nv, uint32_t ranks) {
+            const int64_t col = (int64_t)__shfl_sync(BN_FULL, t, u) * BN_TILE + 4 * lane, r = row0 + __shfl_sync(BN_FULL, sub, u);
+            if (!nv) return;
+            const uint32_t b = ldg_stream_u32(a.raw + (a.ids ? srow : r) * K + col);
+            const uint32_t e0 = tbl[ranks & 0xFFu], e1 = tbl[(ranks >> 8) & 0xFFu], e2 = tbl[(ranks >> 16) & 0xFFu], e3 = tbl[ranks >> 24];
+            *reinterpret_cast<uint2 *>(a.out + r * K + col) = make_uint2((__byte_perm(b, 0u, 0x1100) & 0x807F807Fu) | (e0 << 7) | (e1 << 23), (__byte_perm(b, 0u, 0x3322) & 0x807F807Fu) | (e2 << 7) | (e3 << 23));
           });
         }
         from = to;

@@ -354,6 +354,105 @@ def test_streams_on_any_word(N, K, kind, shift):
         assert torch.equal(a, b)
 
 
+def some_heavy_tiles(rng, N, K):
+    """Ordinary words, with random words, forty equally frequent exponents or lone exponents of any
+    size in one tile of thirty-two each: a stream of fewer than four bits a weight."""
+    u, T = weights(rng, (N, K), escapes=False), -(-K // 128)
+    kind = np.repeat(rng.integers(0, 32, (N, T)), 128, axis=1)[:, :K]
+    e = np.where(kind == 1, rng.integers(100, 140, (N, K)), np.where(rng.random((N, K)) < 0.05, rng.integers(0, 256, (N, K)), u >> 7 & 0xFF))
+    w = ((e << 7) | (u & 0x807F)).astype(np.uint16)
+    return np.where(kind == 0, rng.integers(0, 1 << 16, (N, K)).astype(np.uint16), np.where(kind <= 2, w, u))
+
+
+@pytest.mark.parametrize("N,K", [(33001, 4), (17001, 132), (11003, 260), (70, 1000), (33, 2048), (9, 2052), (40, 4096), (11, 4100), (3, 12296)])
+def test_thread_per_tile_escapes(N, K):
+    """Tiles of every k with many escapes among ordinary ones, 1 to 97 tiles a row: file arrays, BF16
+    rows and R4 arrays (each alone would be a stream for the decoder with a warp per row)."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+
+    u = some_heavy_tiles(np.random.default_rng(N + K), N, K)
+    p = packed_arrays(u)
+    assert len(p["bits"]) * 32 < N * (4.5 * K + 32) and (N * K < 100_000 or set(np.unique(p["meta"] & 3)) >= {0, 1, 2, 3})
+    enc = ck.rice_encode(dev(u))
+    for key in ("meta", "bits", "roff"):
+        assert np.array_equal(enc[key].cpu().numpy().view(p[key].dtype).reshape(-1), p[key].reshape(-1)), key
+    a, want = r4.transcode(p), o.pack_r4(u)
+    for key in ("codes", "flags", "esc", "row_esc"):
+        assert np.array_equal(a[key].cpu().numpy().view(want[key].dtype).reshape(-1), want[key].reshape(-1)), key
+    d = {k: ck.to_device(p[k]) for k in ("raw", "table", "meta", "bits", "roff")}
+    out, rend = ck.rice_unpack(d["meta"].reshape(-1), d["bits"], d["roff"], d["table"], d["raw"], N, K)
+    assert np.array_equal(words(out), u)
+    assert np.array_equal(rend.cpu().numpy().view(np.uint32), np.append(p["roff"][1:], np.uint32(len(p["bits"]))))
+
+
+@pytest.mark.parametrize("N,K", [(64, 2048), (2048, 1024), (30000, 128)])
+@pytest.mark.parametrize("kind", ["uniform", "geometric", "flat", "spread", "mixed"])
+def test_streams_full_of_escapes(N, K, kind):
+    """Streams in which many or nearly all weights escape (random words, geometric ranks, forty equally
+    frequent exponents, one weight in twenty of any exponent, such tiles among ordinary ones): BF16
+    rows and R4 arrays as the decoder with a warp per row gives them (which takes raw bytes and codes
+    off their boundary), in no more than twice its time."""
+    from binade_b200.cuda import kernels as ck
+
+    rng = np.random.default_rng(N + len(kind))
+    if kind == "geometric":
+        e = np.minimum(rng.geometric(0.02, (N, K)), 254)
+    elif kind == "flat":
+        e = rng.integers(100, 140, (N, K))
+    else:
+        e = np.where(rng.random((N, K)) < 0.05, rng.integers(0, 256, (N, K)), rng.integers(118, 126, (N, K)))
+    u = ((e << 7) | rng.integers(0, 128, (N, K))).astype(np.uint16)
+    if kind == "uniform":
+        u = rng.integers(0, 1 << 16, (N, K)).astype(np.uint16)
+    elif kind == "mixed":
+        u = some_heavy_tiles(rng, N, K)
+    p, T = packed_arrays(u), -(-K // 128)
+    d = {k: ck.to_device(p[k]).reshape(-1) for k in ("raw", "table", "meta", "bits", "roff")}
+    stream = (ck._p(d["meta"]), ck._p(d["bits"]), d["bits"].numel(), ck._p(d["roff"]), ck._p(d["table"]))
+    off = torch.empty(N * K + 16, dtype=torch.uint8, device="cuda")[4 : 4 + N * K].copy_(d["raw"])
+    flags, esc = torch.empty(N * T, dtype=torch.uint8, device="cuda"), torch.zeros(N * K, dtype=torch.uint8, device="cuda")
+    cnt, at, ctr = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (N, N, 8))
+    out, rend = torch.empty((N, K), dtype=torch.bfloat16, device="cuda"), torch.empty(N, dtype=torch.int32, device="cuda")
+
+    def run(op, aligned):
+        if op == "unpack":
+            raw = d["raw"] if aligned else off
+            return (lambda: ck._call("bn_rice_unpack", *stream, ck._p(raw), N, K, ck._p(out), ck._p(rend))), lambda: [out.view(torch.int16).clone(), rend.clone()]
+        codes = torch.empty(N * T * 32 + 2, dtype=torch.int16, device="cuda")[0 if aligned else 2 :][: N * T * 32]
+
+        def arrays():
+            rows, run_bytes = torch.empty_like(cnt), torch.empty(int(ctr[2]) + 1, dtype=torch.uint8, device="cuda")
+            ck._call("bn_r4_finish", ck._p(cnt), ck._p(esc), ck._p(at), N, ck._p(rows), ck._p(run_bytes), run_bytes.numel())
+            return [codes.clone(), flags.clone(), cnt.clone(), rows, run_bytes, ctr[1:3].clone()]
+
+        return (lambda: ck._call("bn_rice_to_r4", *stream, N, K, ck._p(codes), ck._p(flags), ck._p(cnt), ck._p(esc), N * K, ck._p(at), ck._p(ctr))), arrays
+
+    def microseconds(call):
+        call()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = float("inf")
+        for _ in range(5):
+            a.record()
+            for _ in range(4):
+                call()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 250)
+        return best
+
+    for op in ("unpack", "to_r4"):
+        (fast, got), (rows, want) = run(op, True), run(op, False)
+        fast()
+        results = got()
+        rows()
+        for x, y in zip(results, want()):
+            assert torch.equal(x, y), op
+        if op == "unpack":
+            assert np.array_equal(results[0].cpu().numpy().view(np.uint16), u)
+        assert microseconds(fast) <= 2 * microseconds(rows), op
+
+
 def test_transcode_all_escapes_grows_scratch():
     """Uniform exponents: nearly every weight escapes, far beyond the default scratch size."""
     from binade_b200.cuda import r4
