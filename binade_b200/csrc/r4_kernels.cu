@@ -435,10 +435,24 @@ extern "C" int bn_r4_rows(const uint16_t *x, int64_t x_stride, const bn_r4 *w, i
     int e = pass(0, M);
     // long rows, whose x does not fit beside the rings: passes over the weights by the most rows that
     // do fit still beat one pass of the plain-load kernel (3840 x 15360: 81 us against 583 at four
-    // rows). Where no pass fits (more than 200 tiles, unaligned arrays) that one pass it is.
+    // rows)
     for (int64_t part = M > 4 ? 4 : 2; e == -1 && part >= 2 && part < M; part /= 2) {
       e = pass(0, part);
       if (e == BN_OK) return bn_r4_rows(x + part * x_stride, x_stride, w, M - part, N, K, y + part * y_stride, y_stride, stream);
+    }
+    // rows of more than 200 tiles are beyond the rings: one input row after the other through the
+    // one-row kernel (4096 x 28672: 53 us each, against 1200 for three in one plain-load pass, 2460 for eight)
+    if (e == -1 && tiles(K) > 200 && K % 16 == 0 && x_stride % 8 == 0 && !((reinterpret_cast<uintptr_t>(w->raw) | reinterpret_cast<uintptr_t>(w->codes) | reinterpret_cast<uintptr_t>(x)) & 15)) {
+      for (int64_t m = 0; m < M; m++)
+        if (int e1 = bn_r4_rows(x + m * x_stride, x_stride, w, 1, N, K, y + m * y_stride, y_stride, stream)) return e1;
+      return BN_OK;
+    }
+    // plain loads: eight rows of x in fp32 are staged in chunks from 25 tiles on, where two passes by four
+    // rows are as fast or faster (us, one / two: 4096 x 3840 255 / 115, 15360 x 3840 152 / 128, 1000 x 3844
+    // 95 / 98; 8192 x 2048, not in chunks, 43 / 58)
+    if (e == -1 && M > 4 && tiles(K) > 24) {
+      if (int e1 = bn_r4_rows(x, x_stride, w, 4, N, K, y, y_stride, stream)) return e1;
+      return bn_r4_rows(x + 4 * x_stride, x_stride, w, M - 4, N, K, y + 4 * y_stride, y_stride, stream);
     }
     if (e >= 0) return e;
   }

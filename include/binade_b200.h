@@ -227,8 +227,8 @@ int bn_rice_lookup(const uint8_t *meta, const uint32_t *bits, uint64_t nwords, c
  * their products (fused multiply-add) for t then j ascending; columns >= K are skipped; lanes
  * combine with strides 16, 8, 4, 2, 1; one round-to-nearest-even to BF16. M = 1 replaces
  * r4_matvec, binade/mlx/cuda_kernels.py:118-130 (same order for K % 128 == 0). The weights are
- * read once, but for M = 3..8 on rows so long that X does not fit on chip beside the copies in
- * flight: there once per two or four rows. x_stride / y_stride: elements between rows of X / Y. Any
+ * read once, but for M <= 8 on rows so long that X does not fit on chip (beside the copies in
+ * flight): there once per one, two or four rows. x_stride / y_stride: elements between rows of X / Y. Any
  * alignment of x is served; the fastest kernels need x and the raw / codes arrays on 16-byte
  * boundaries and K % 16 == 0 (other calls run a plain-load kernel with the same results). */
 int bn_r4_rows(const uint16_t *x, int64_t x_stride, const bn_r4 *w, int64_t M, int64_t N, int64_t K,

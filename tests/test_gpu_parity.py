@@ -856,11 +856,12 @@ def test_rows_of_many_row_matrices(N, K, M):
         assert np.array_equal(got[i], words(m(x[i]))), i
 
 
-@pytest.mark.parametrize("N,K,M,shift,passes", [(64, 25616, 3, 0, 1), (64, 25616, 8, 0, 1), (64, 28672, 4, 0, 1), (96, 1024, 4, 1, 1), (4100, 1024, 8, 3, 1), (64, 264, 8, 0, 1), (3840, 15360, 4, 0, 2), (3840, 15360, 8, 0, 4)])
+@pytest.mark.parametrize("N,K,M,shift,passes", [(64, 25616, 2, 0, 2), (64, 25616, 3, 0, 3), (64, 28672, 8, 0, 8), (64, 28672, 4, 1, 1), (96, 1024, 4, 1, 1), (4100, 1024, 8, 3, 1), (64, 264, 8, 0, 1), (64, 3844, 8, 0, 2), (64, 3840, 7, 1, 2), (64, 3072, 8, 1, 1), (3840, 15360, 4, 0, 2), (3840, 15360, 8, 0, 4)])
 def test_passes_over_the_weights(N, K, M, shift, passes):
-    """Three to eight input rows are cut only where the parts fit a kernel with rings: rows of more
-    than 200 tiles, an x off its 16-byte boundary and K % 16 != 0 take one pass, long rows that
-    do not fit beside x one per two rows; the bits are the one-row kernel's."""
+    """Two to eight input rows are cut only where the parts fit a faster kernel: long rows that do not
+    fit beside x take one pass per two rows, rows of more than 200 tiles one per row; an x off its
+    16-byte boundary and K % 16 != 0 take a single one, two from five rows and 25 tiles on; the bits are the
+    one-row kernel's."""
     from binade_b200.cuda import kernels as ck
     from binade_b200.cuda import r4
 
