@@ -8,7 +8,7 @@
 // The bit offset of a lane inside a plane is the number of alive weights before it: a warp
 // prefix sum over per-lane alive counts, done with three ballots. These kernels take what the faster
 // decoder with a thread per tile (rice_tiles.cu) does not: ranks, K % 4 != 0, raw bytes and BF16
-// rows off a 16-byte boundary, streams full of escapes, and format 1.
+// rows off a 16-byte boundary, few short rows, streams full of escapes, and format 1.
 #include <atomic>
 
 #include "rice.cuh"
@@ -532,12 +532,23 @@ static int rice_grid(int64_t R) {
 // 2.6 bits). A word a row is left out of the count: rows start on words.
 static bool heavy_stream(const RiceArgs &a) { return (double)a.nwords * 32 > (double)(a.ids ? a.rows : a.R) * (4.5 * (double)a.K + 32); }
 
-// A thread per tile where the arrays allow it (K % 4 == 0, codes on 8 bytes); heavy streams and what
-// else it does not take by four rows a warp when the matrix has rows for that on every SM, two from
+// Few short rows: a warp per row is done before the other decoder's second launch has its 64 KB table (us,
+// warp per row / thread per tile, BF16 rows of 128 weights: 1000 rows 10.9 / 14.2, 16000 16.6 / 20.7,
+// 32000 30 / 27; of 260: 8000 rows 23 / 25, 16000 37 / 27; of 704: 300 rows 16.5 / 18.6, 4000 24.9 / 24.9; R4
+// arrays alike). Looked-up rows are a task of that decoder each, however short (128: 64000 rows
+// 56 / 134; 512: 32000 rows 89 / 94, 64000 181 / 173; 704: 64 rows 16.5 / 15.2, 300 16.6 / 18.6, 4000 24.8 /
+// 24.8, 8000 39 / 37).
+static bool few_tiles(const RiceArgs &a) {
+  if (a.ids) return a.T < 6 ? a.R * (2 * a.T - 7) < 32768 : a.T < 8 && a.R >= 150 && a.R * (2 * a.T - 7) < 32768;
+  return a.T < 8 && a.R * a.T < 24576;
+}
+
+// A thread per tile where the arrays allow it (K % 4 == 0, codes on 8 bytes); few short rows, heavy
+// streams and what else it does not take by four rows a warp when the matrix has rows for that on every SM, two from
 // half of that, else one row a warp: fewer instructions per row against fewer warps to hide a plane
 // step's latency (us, thread per tile / this: random words 100000 x 128 309 / 167, 4096 x 3840 470 / 380).
 static int launch_rice_r4(const RiceArgs &a, cudaStream_t s) {
-  if (!heavy_stream(a)) {
+  if (!few_tiles(a) && !heavy_stream(a)) {
     const int e = rice_tiles_r4(a, s);
     if (e != -1) return e;
   }
@@ -560,7 +571,7 @@ static int launch_rice_r4(const RiceArgs &a, cudaStream_t s) {
 
 // BF16 rows alike (K % 4 == 0, raw bytes and rows on 16 bytes).
 static int launch_rice_unpack(const RiceArgs &a, cudaStream_t s) {
-  const int e = heavy_stream(a) ? -1 : rice_tiles_unpack(a, s);
+  const int e = few_tiles(a) || heavy_stream(a) ? -1 : rice_tiles_unpack(a, s);
   if (e != -1) return e;
   rice_kernel<RICE_UNPACK><<<rice_grid(a.R), RICE_THREADS, 0, s>>>(a);
   return launched("rice_kernel<unpack>");

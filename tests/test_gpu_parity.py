@@ -354,6 +354,27 @@ def test_streams_on_any_word(N, K, kind, shift):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("N,K,rows_a_warp", [(1, 128, True), (64, 128, True), (1000, 128, True), (24575, 128, True), (24576, 128, False), (5000, 260, True), (9000, 260, False), (300, 704, True), (5000, 704, False), (1, 1000, False), (64, 1024, False), (1, 3840, False)])
+def test_small_streams(N, K, rows_a_warp):
+    """Few short rows are one launch of the decoder with a warp per row, the others two of the one
+    with a thread per tile; looked-up rows follow a line of their own."""
+    from binade_b200.cuda import kernels as ck
+
+    u = weights(np.random.default_rng(N + K), (N, K), escapes=False)
+    p = packed_arrays(u)
+    d = {k: ck.to_device(p[k]).reshape(-1) for k in ("raw", "table", "meta", "bits", "roff")}
+    read = lambda: ck.rice_unpack(d["meta"], d["bits"], d["roff"], d["table"], d["raw"], N, K)  # noqa: E731
+    assert launches(read) == (1 if rows_a_warp else 2)
+    assert np.array_equal(words(read()[0]), u)
+    for n in (1, 4000, 12000):
+        ids = torch.randint(0, N + 1, (n,), generator=torch.Generator().manual_seed(n), dtype=torch.int32).cuda()
+        look = lambda: ck.rice_lookup(d["meta"], d["bits"], d["roff"], d["table"], d["raw"], N, K, ids)  # noqa: E731
+        T = -(-K // 128)
+        assert launches(look) == (1 if T < 4 or (T < 6 and n <= 4000) or (T < 8 and n == 4000) else 2)
+        i = ids.cpu().numpy()
+        assert np.array_equal(words(look()), np.where((i < N)[:, None], u[np.minimum(i, N - 1)], np.uint16(0)))
+
+
 def some_heavy_tiles(rng, N, K):
     """Ordinary words, with random words, forty equally frequent exponents or lone exponents of any
     size in one tile of thirty-two each: a stream of fewer than four bits a weight."""
