@@ -480,7 +480,11 @@ EncShape enc_shape(int64_t R, int T) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int rows = T > 16 ? 1 : 32 / T;
+  // as many rows a task as keep every warp of the write at one task, up to the task's 32 tiles: tiles of
+  // many planes fill the window six at a time, and a warp with 32 of them takes six turns while others
+  // idle (random words, us: 64 x 128 144 -> 67, 1000 x 128 161 -> 69; ordinary words 72 -> 67)
+  const int64_t all_warps = (int64_t)sms * EN_WRITE_WARPS;
+  const int rows = T > 16 ? 1 : (int)max((int64_t)1, min((int64_t)(32 / T), (R + all_warps - 1) / all_warps));
   const int64_t tasks = (R + rows - 1) / rows;
   return {(unsigned)min(tasks, (int64_t)sms), rows};
 }

@@ -375,6 +375,33 @@ def test_small_streams(N, K, rows_a_warp):
         assert np.array_equal(words(look()), np.where((i < N)[:, None], u[np.minimum(i, N - 1)], np.uint16(0)))
 
 
+@pytest.mark.parametrize("N,K", [(1, 128), (3, 500), (1000, 128), (2961, 260), (5000, 260), (6001, 640), (23681, 512)])
+def test_encode_spreads_short_rows(N, K):
+    """Plan and write deal short rows out over all multiprocessors before a warp gets several of
+    them, and the arrays are the host encoder's either way (around one row a warp, several rows a
+    task, a task cut short)."""
+    from binade_b200.cuda import kernels as ck
+    from cuda.bindings import driver
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    u = np.random.default_rng(N + K).integers(0, 1 << 16, (N, K)).astype(np.uint16)
+    p, T = packed_arrays(u), -(-K // 128)
+    w, rank = dev(u), torch.arange(256, dtype=torch.uint8, device="cuda")
+    meta, words_a_row, roff, total = (torch.empty(n, dtype=t, device="cuda") for n, t in ((N * T, torch.uint8), (N, torch.int32), (N, torch.int32), (1, torch.int64)))
+    plan = lambda: ck._call("bn_rice_encode_plan", ck._p(w), ck._p(rank), N, K, ck._p(meta), ck._p(words_a_row), ck._p(roff), ck._p(total))  # noqa: E731
+    plan()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        plan()
+    status, nodes, _ = driver.cuGraphGetNodes(driver.CUgraph(graph.raw_cuda_graph()), 2)
+    assert status == driver.CUresult.CUDA_SUCCESS
+    status, params = driver.cuGraphKernelNodeGetParams(nodes[0])
+    assert status == driver.CUresult.CUDA_SUCCESS and params.gridDimX == min(N, sms)
+    enc = ck.rice_encode(w)
+    for key in ("table", "meta", "bits", "roff"):
+        assert np.array_equal(enc[key].cpu().numpy().view(p[key].dtype).reshape(-1), p[key].reshape(-1)), key
+
+
 def some_heavy_tiles(rng, N, K):
     """Ordinary words, with random words, forty equally frequent exponents or lone exponents of any
     size in one tile of thirty-two each: a stream of fewer than four bits a weight."""
