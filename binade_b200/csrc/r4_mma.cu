@@ -12,7 +12,9 @@
 //   r4_mma_oct_kernel  K % 16 == 0: up to 26 warps, eight threads per weight row, private
 //                      cp.async rings (the batch-1 matvec's decode, oct.cuh)
 //   r4_mma_kernel      the rest (many input rows with many weight rows a block, where the other's
-//                      stages do not fit; K % 16 == 8; unaligned arrays): 14 warps, a warp per row and stage, 8 rows each, raw bytes and codes fetched two stages ahead into registers
+//                      stages do not fit; rows that fill fewer waves of its larger blocks; K % 16 == 8;
+//                      unaligned arrays): 14 warps, a warp per row and stage, 8 rows each, raw bytes
+//                      and codes fetched two stages ahead into registers
 // The weights are read once whatever M. The sum over K is the hardware's: 16 k per MMA step, in
 // order, from zero, in fp32: not the documented lane order of the one-row kernels, but the
 // order of cuBLAS's BF16 GEMM on this GPU, whose outputs this kernel reproduces bit for bit;
@@ -674,8 +676,14 @@ int mma_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int
   if (encode(&x_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(x), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return fail(BN_ERR_CUDA, "cuTensorMapEncodeTiled failed for the input rows");
   const uint32_t fixed = 1024 + LUT_WORDS * 4 + MMA_BARS;  // alignment slack, pair table, barriers
-  if (K % 16 == 0 && !(((uintptr_t)w->raw | (uintptr_t)w->codes) & 15)) {
-    constexpr int ow = MMA_OCT_WARPS;
+  constexpr int ow = MMA_OCT_WARPS, dw = MMA_DECODE_WARPS, rpw = MMA_RPW;
+  // blocks of 104 rows with eight threads per row, of 112 with a warp per row: where the larger ones
+  // need fewer waves, the slower decode may still be ahead. A wave takes (us, 2048 columns, eight
+  // threads / a warp) 20 / 26 with up to 64 input rows, 22 / 27 with 96, 26 / 27 with 144, 25 / 29 with 192:
+  // 15984 rows (two waves or one) 39 / 28 at 17 input rows, 53 / 31 at 144, 50 / 31 at 192.
+  auto waves = [&](int64_t most) { return (N + mma_sms() * most - 1) / (mma_sms() * most); };
+  const bool larger_blocks = waves(dw * rpw) * (a.BN <= 96 ? 25 : 22) < waves(ow * 4) * 20;
+  if (K % 16 == 0 && !(((uintptr_t)w->raw | (uintptr_t)w->codes) & 15) && !larger_blocks) {
     const bool cols = w->esc_cols && w->col_esc && !(((uintptr_t)w->esc_cols | (uintptr_t)w->col_esc) & 3);
     int64_t rows = (N + mma_sms() - 1) / mma_sms();
     rows = (rows + 3) / 4 * 4;
@@ -706,7 +714,6 @@ int mma_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int
   }
   const uint32_t per_stage = MMA_A_STAGE + (uint32_t)a.BN * MMA_BK * 2u;
   // an equal share of the rows for every SM, in whole warps' worth of rows
-  constexpr int dw = MMA_DECODE_WARPS, rpw = MMA_RPW;
   int64_t rows = (N + mma_sms() - 1) / mma_sms();
   rows = (rows + rpw - 1) / rpw * rpw;
   if (rows > dw * rpw) rows = dw * rpw;

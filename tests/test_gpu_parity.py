@@ -1077,6 +1077,34 @@ def test_mma_tile_phases(N, K, M, density):
     assert bool(((got.double() - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("rows,M,waves", [(104, 144, 1), (108, 5, 1), (108, 144, 1), (112, 192, 1), (113, 160, 2), (216, 100, 2), (216, 176, 2), (224, 64, 2), (936, 17, 9)])
+def test_mma_waves(rows, M, waves):
+    """Weight rows just past a wave of blocks (`rows` an SM): no wave more than the larger blocks need,
+    unless the faster decode makes up for it; the product's bits either way."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+    from cuda.bindings import driver
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    N, K = sms * rows, 128
+    g = torch.Generator(device="cuda").manual_seed(rows + M)
+    m = r4.R4Linear(r4.from_dense((torch.randn((N, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)))
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    got = m.mma_rows(x)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        m.mma_rows(x)
+    status, nodes, _ = driver.cuGraphGetNodes(driver.CUgraph(graph.raw_cuda_graph()), 1)
+    assert status == driver.CUresult.CUDA_SUCCESS
+    status, params = driver.cuGraphKernelNodeGetParams(nodes[0])
+    assert status == driver.CUresult.CUDA_SUCCESS
+    assert -(-params.gridDimX // sms) == waves
+    half = N // 2  # blocks of other rows, and of the other kernel where those are one wave
+    part = {k: (v[:half] if v.dim() > 1 else v) for k, v in m._a.items() if k in ("raw",)}
+    top = dict(m._a, raw=part["raw"], codes=m._a["codes"][: half * 32], flags=m._a["flags"][:half], row_esc=m._a["row_esc"][:half], col_esc=m._a["col_esc"][:half])
+    assert np.array_equal(words(ck.r4_mma(top, x, half, K)), words(got[:, :half]))
+
+
 @pytest.mark.parametrize("N,K", [(384, 1024), (520, 3840), (256, 15360), (128, 16384)])
 def test_mma_rows_in_the_order_of_cublas(N, K):
     """Split-K in the kernel (every slice from zero in its own accumulator, fp32 sums added in
