@@ -370,9 +370,11 @@ __global__ void __launch_bounds__((DW + 1) * 32, 1) r4_mma_kernel(const __grid_c
 //             order of k. A thread's escape cursors still have to pass the tiles of the other
 //             phases; only code words of tiles that its row flags matter for that, and those
 //             are copied into the ring and counted
-//   A stages  hold the block's rows only: the MMA reads its M rows from their start, the rest of
-//             which are other stages' bytes and end in accumulator lanes that nobody reads (the
-//             window goes on past the last stage). Smaller stages mean more of them
+//   A stages  hold the block's rows only where that makes room for another stage: the MMA reads its M
+//             rows from their start, the rest of which are other stages' bytes and end in accumulator
+//             lanes that nobody reads (the window goes on past the last stage). Where as many stages
+//             of 128 rows fit, they have those: 15360 x 3840 with 128 input rows 46.7 -> 42.6 us, 144
+//             47.4 -> 42.9 (of 64 rows: no gain, and escapes want the L1 that this takes)
 //   M = 64    for blocks of up to 64 rows
 //   MMA warp  issues through elect.sync and asks for the next stage before it issues (waiting
 //             stages and uniform operands took 1000 of 1500 cycles a tile)
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__((DW + 1) * 32, 1) r4_mma_kernel(const __grid_c
 // at 128, 133 -> 92 at 200; 15360 rows out of 3840 columns 37.9 -> 33.0, 43.8 -> 44.4, 50.8 -> 50.3.
 struct MmaOctPlan {
   int phases, groups;   // tile phases; row groups of four (groups * phases decode warps)
-  int a_rows;           // rows of an A stage: the block's, rounded up to 8
+  int a_rows;           // rows of an A stage: the block's, rounded up to 8, or 128
   int m;                // MMA M: 64 for up to 64 rows (half the A bytes to read per MMA, which is what few input rows cost), else 128
   int slots;            // stages
   uint32_t ring_slot;   // bytes of a warp's ring slot: 512 raw, 256 codes, 256 for the codes of each skipped tile
@@ -692,7 +694,7 @@ int mma_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int
     MmaOctPlan pl{};
     b.rows = (int)rows, pl.groups = (int)rows / 4, pl.a_rows = (int)(rows + 7) / 8 * 8, pl.m = rows <= 64 ? 64 : MMA_BM;
     pl.flag_words = (uint32_t)(a.T + 31) / 32 + 1;
-    const uint32_t stage = (uint32_t)(pl.a_rows + a.BN) * 256u;
+    const uint32_t small = (uint32_t)(pl.a_rows + a.BN) * 256u, full = (uint32_t)(pl.m + a.BN) * 256u;
     // as many phases as the warps allow (at most four: every phase adds 256 bytes to a ring slot)
     // with at least one stage more than phases. Measured with 1 / 2 / 3 phases (us): 28 rows a
     // block, 15360 columns, 17 input rows 67.6 / 63.1 / 55.8; 16 rows a block, 3840 columns 21.1 /
@@ -702,8 +704,10 @@ int mma_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int
       pl.phases = phases, pl.ring_slot = 512u + 256u * phases;
       const uint32_t rings = (uint32_t)(pl.groups * phases * MMA_RING) * pl.ring_slot, flags = (phases > 1 ? (uint32_t)rows * pl.flag_words * 4u : 0u) + 128u;
       const uint32_t left = fixed + flags + rings < MMA_SMEM_MAX ? MMA_SMEM_MAX - fixed - flags - rings : 0u;
-      b.stages = min(8, (int)(left / stage));
+      b.stages = min(8, (int)(left / small));
       if (b.stages < (phases > 1 ? phases + 1 : 2)) continue;
+      const uint32_t stage = pl.m == MMA_BM && (uint32_t)b.stages * full <= left ? full : small;
+      if (stage == full) pl.a_rows = pl.m;
       const uint32_t smem = fixed + flags + rings + (uint32_t)b.stages * stage;
       const unsigned grid = (unsigned)((N + rows - 1) / rows), threads = 32u * (unsigned)max(4, pl.groups * phases + 2);
       auto kern = phases > 1 ? r4_mma_oct_kernel<ow, MMA_RING, true, true> : cols ? r4_mma_oct_kernel<ow, MMA_RING, true, false> : r4_mma_oct_kernel<ow, MMA_RING, false, false>;
