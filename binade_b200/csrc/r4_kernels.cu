@@ -17,8 +17,7 @@ __device__ __forceinline__ float hi_f32(uint32_t w) { return __uint_as_float(w &
 // R4 -> dense BF16
 // ---------------------------------------------------------------------------------------------
 constexpr int DEC_THREADS = 256;
-constexpr int DEC_WIDE_WARPS = 13;  // most warps of a block of the wide decode (two blocks an SM)
-constexpr int DEC_AHEAD = 3;        // tiles of a row in flight per thread there
+constexpr int DEC_WIDE_WARPS = 13;  // most warps of a block of the wide decode that have rows
 
 __global__ void __launch_bounds__(DEC_THREADS) r4_decode_kernel(bn_r4 w, int64_t N, int64_t K, int T, int64_t NB, int64_t RS, int64_t R0, const uint32_t *__restrict__ ids, int64_t rows, uint16_t *__restrict__ out) {
   extern __shared__ uint32_t lut[];
@@ -60,11 +59,12 @@ __global__ void __launch_bounds__(DEC_THREADS) r4_decode_kernel(bn_r4 w, int64_t
 // bytes of code words of a tile with one load each, decodes 16 weights and stores 32 bytes, so a
 // warp instruction moves four rows' worth; escapes by column streams when the matrix carries
 // them. About a third of the instructions per weight of the kernel above. A thread's bytes are
-// fetched DEC_AHEAD tiles ahead (one memory latency per tile bounded the kernel), and two blocks an
+// fetched AHEAD tiles ahead (one memory latency per tile bounded the kernel), and PER_SM blocks an
 // SM share the rows evenly (blocks of eight warps left every fourth SM with a third more rows): a
 // product of 2048 input rows with 15360 x 3840, which rebuilds the weight first, 238.0 -> 233.4 us.
-template <bool COLS>
-__global__ void __launch_bounds__(DEC_WIDE_WARPS * 32, 2) r4_decode_wide_kernel(bn_r4 w, int64_t N, int64_t K, int T, int64_t NB, int64_t RS, int64_t R0, uint16_t *__restrict__ out) {
+// The first `warps` warps of a block have rows, the others help with the table.
+template <bool COLS, int AHEAD, int PER_SM>
+__global__ void __launch_bounds__(DEC_WIDE_WARPS * 32, PER_SM) r4_decode_wide_kernel(bn_r4 w, int64_t N, int64_t K, int T, int64_t NB, int64_t RS, int64_t R0, int warps, uint16_t *__restrict__ out) {
   constexpr int R = 4;
   using Geo = OctGeom<R>;
   extern __shared__ uint32_t lut[];
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(DEC_WIDE_WARPS * 32, 2) r4_decode_wide_kernel(
   me.esc = w.esc, me.esc_cap = w.n_esc + 1, me.esc_cols = w.esc_cols;
   const bool partial = (K & 127) != 0;
   const uint32_t pmax = (uint32_t)(K & 127) / 16u;
-  const int warps = (int)(blockDim.x >> 5);
+  if ((int)(threadIdx.x >> 5) >= warps) return;
   for (int64_t g = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); g * R < N; g += (int64_t)gridDim.x * warps) {
     const int64_t orow = g * R + grp;
     const bool valid = orow < N;
@@ -98,19 +98,19 @@ __global__ void __launch_bounds__(DEC_WIDE_WARPS * 32, 2) r4_decode_wide_kernel(
       ew.base = epos & ~3u;
       ew.word = window_load(me.esc, me.esc_cap, ew.base + p * 4u);
     }
-    // a thread's bytes of the next DEC_AHEAD tiles wait in registers
-    uint4 ahead_raw[DEC_AHEAD];
-    uint2 ahead_codes[DEC_AHEAD];
+    // a thread's bytes of the next AHEAD tiles wait in registers
+    uint4 ahead_raw[AHEAD];
+    uint2 ahead_codes[AHEAD];
     auto fetch = [&](int t, uint4 &rr, uint2 &c2) {
       rr = t < T && (!(partial && t == T - 1) || p < pmax) ? __ldcs(reinterpret_cast<const uint4 *>(raw + (int64_t)t * 128)) : make_uint4(0, 0, 0, 0);
       c2 = t < T ? __ldcs(reinterpret_cast<const uint2 *>(codes + (int64_t)t * 64)) : make_uint2(0, 0);
     };
 #pragma unroll
-    for (int u = 0; u < DEC_AHEAD; u++) fetch(u, ahead_raw[u], ahead_codes[u]);
+    for (int u = 0; u < AHEAD; u++) fetch(u, ahead_raw[u], ahead_codes[u]);
     uint32_t fm = 0, nflag = (int)p < T ? (uint32_t)__ldg(flags + p) : 0u;  // this thread's flag byte of the next block of eight tiles
-    for (int t0 = 0; t0 < T; t0 += DEC_AHEAD)
+    for (int t0 = 0; t0 < T; t0 += AHEAD)
 #pragma unroll
-    for (int u = 0; u < DEC_AHEAD; u++) {
+    for (int u = 0; u < AHEAD; u++) {
       const int t = t0 + u;
       if (t >= T) break;
       if ((t & 7) == 0) {  // the flag bytes of eight tiles, folded over the warp's four rows
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(DEC_WIDE_WARPS * 32, 2) r4_decode_wide_kernel(
       const bool live = !(partial && t == T - 1) || p < pmax;
       const uint4 rr = ahead_raw[u];
       const uint2 c2 = ahead_codes[u];
-      fetch(t + DEC_AHEAD, ahead_raw[u], ahead_codes[u]);
+      fetch(t + AHEAD, ahead_raw[u], ahead_codes[u]);
       const uint32_t r4w[4] = {rr.x, rr.y, rr.z, rr.w}, cc[2] = {c2.x, c2.y};
       uint32_t wv[2 * R];
 #pragma unroll
@@ -365,13 +365,18 @@ extern "C" int bn_r4_decode(const bn_r4 *w, int64_t N, int64_t K, int64_t NB, in
   const size_t smem = LUT_WORDS * 4;
   const int warps = DEC_THREADS / 32;
   if (K % 16 == 0 && !((reinterpret_cast<uintptr_t>(w->raw) | reinterpret_cast<uintptr_t>(w->codes) | reinterpret_cast<uintptr_t>(out)) & 15) && !((reinterpret_cast<uintptr_t>(w->esc) | reinterpret_cast<uintptr_t>(w->esc_cols) | reinterpret_cast<uintptr_t>(w->col_esc)) & 3)) {
-    // two blocks an SM, with as many warps as spread the groups of four rows evenly over them
-    const int64_t groups = (N + 3) / 4, most = (int64_t)sm_count() * 2, rounds = (groups + most * DEC_WIDE_WARPS - 1) / (most * DEC_WIDE_WARPS);
-    const int64_t wide = (groups + most * rounds - 1) / (most * rounds), blocks = (groups + wide - 1) / wide < most ? (groups + wide - 1) / wide : most;
-    const bool cols = w->esc_cols && w->col_esc;
-    auto kern = cols ? r4_decode_wide_kernel<true> : r4_decode_wide_kernel<false>;
+    // Two blocks an SM, or three with two tiles ahead instead of three where the rows then take fewer
+    // rounds (us, 2048 columns, two / three blocks: 15312 rows 23 / 27, 16792 36 / 30, 22712 44 / 37, 24192
+    // 45 / 52, 31592 58 / 56); as many warps as spread the groups of four rows evenly over them, and at
+    // least eight for the table (1000 x 15360 81 -> 74)
+    const int64_t groups = (N + 3) / 4;
+    auto rounds = [&](int64_t blocks) { return (groups + blocks * DEC_WIDE_WARPS - 1) / (blocks * DEC_WIDE_WARPS); };
+    const int64_t two = (int64_t)sm_count() * 2, three = (int64_t)sm_count() * 3;
+    const bool cols = w->esc_cols && w->col_esc, third = rounds(three) < rounds(two);
+    const int64_t most = (third ? three : two) * rounds(third ? three : two), wide = (groups + most - 1) / most, fill = (groups + wide - 1) / wide;
+    auto kern = third ? (cols ? r4_decode_wide_kernel<true, 2, 3> : r4_decode_wide_kernel<false, 2, 3>) : cols ? r4_decode_wide_kernel<true, 3, 2> : r4_decode_wide_kernel<false, 3, 2>;
     BN_CUDA(allow_smem(kern, smem));
-    kern<<<(unsigned)blocks, (unsigned)wide * 32, smem, (cudaStream_t)stream>>>(*w, N, K, (int)tiles(K), NB, RS, R0, out);
+    kern<<<(unsigned)min(fill, third ? three : two), (unsigned)max((int64_t)8, wide) * 32, smem, (cudaStream_t)stream>>>(*w, N, K, (int)tiles(K), NB, RS, R0, (int)wide, out);
     return launched("r4_decode_wide_kernel");
   }
   BN_CUDA(allow_smem(r4_decode_kernel, smem));
