@@ -700,12 +700,16 @@ int mma_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int
     // block, 15360 columns, 17 input rows 67.6 / 63.1 / 55.8; 16 rows a block, 3840 columns 21.1 /
     // 18.2 / 16.2 (15.7 with four)
     const int most = cols ? max(1, min(4, ow / pl.groups)) : 1;
+    // with half the weights escaped, one after the other in a thread here, four lanes share them there:
+    // one phase only (us, this / a warp per row: 15360 x 3840, 144 input rows, 28 % 102 / 113, 47 % 121 / 112,
+    // 94 % 163 / 112; 4096 x 3840 with 200 rows 47 % 93 / 93, 94 % 118 / 95; several phases, 144 rows, 94 % 69 / 94; blocks of 8 rows, 256 rows 18 / 23)
+    const bool many_escapes = (double)w->n_esc > 0.46 * (double)N * (double)K;
     for (int phases = most; phases >= 1; phases--) {
       pl.phases = phases, pl.ring_slot = 512u + 256u * phases;
       const uint32_t rings = (uint32_t)(pl.groups * phases * MMA_RING) * pl.ring_slot, flags = (phases > 1 ? (uint32_t)rows * pl.flag_words * 4u : 0u) + 128u;
       const uint32_t left = fixed + flags + rings < MMA_SMEM_MAX ? MMA_SMEM_MAX - fixed - flags - rings : 0u;
       b.stages = min(8, (int)(left / small));
-      if (b.stages < (phases > 1 ? phases + 1 : 2)) continue;
+      if (b.stages < (phases > 1 ? phases + 1 : 2) || (phases == 1 && pl.groups > 4 && many_escapes)) continue;
       const uint32_t stage = pl.m == MMA_BM && (uint32_t)b.stages * full <= left ? full : small;
       if (stage == full) pl.a_rows = pl.m;
       const uint32_t smem = fixed + flags + rings + (uint32_t)b.stages * stage;

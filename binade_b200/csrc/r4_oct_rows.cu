@@ -393,6 +393,12 @@ int oct_rows(const bn_r4 *w, const uint16_t *x, int64_t x_stride, int64_t M, int
   // two input rows, that kernel / this: 2048 x 3840 9.9 / 11.1, 3840 x 15360 40.6 / 42.1, 4096 x
   // 3840 14.3 / 11.8, 15360 x 3840 36.1 / 23.4)
   if (N < blocks * 27) return -1;
+  // a thread applies its columns' escapes one after the other, which the few warps of few weight rows do not
+  // hide: from a share of the weights that grows with the rows an SM has, the bulk-copy kernel is faster
+  // (us, this / that with two input rows: 4096 x 3840, a fifth escaped 31 / 35, 28 % 39 / 37; 8192 x 2048, half
+  // 34 / 39, 70 % 44 / 39; 15360 x 3840, 94 % 149 / 172; with eight, half escaped 189 / 179)
+  const double escaped = (double)w->n_esc / ((double)N * (double)K), rows_an_sm = (double)N / (double)blocks;
+  if (escaped > rows_an_sm / 110 || (M > 4 && escaped > 0.5)) return -1;
   return M == 2 ? launch_rows<2, 26>(a, blocks, 1, s) : M <= 4 ? launch_rows<4, 26>(a, blocks, 1, s) : launch_rows<8, 16>(a, blocks, 1, s);
 }
 

@@ -1105,6 +1105,30 @@ def test_mma_waves(rows, M, waves):
     assert np.array_equal(words(ck.r4_mma(top, x, half, K)), words(got[:, :half]))
 
 
+@pytest.mark.parametrize("N,K,share", [(4096, 640, 0.1), (4096, 640, 0.9), (8200, 656, 0.6), (15360, 640, 0.45), (15360, 640, 0.55), (15360, 640, 0.95)])
+def test_products_of_escapes(N, K, share):
+    """Weights of which a tenth to nearly all escape, on either side of the lines where products go
+    to the kernels that share a row's escapes among lanes: two to eight rows have the bits of the one-row
+    kernel, the tensor-core product those of row-ordered escapes on another shape."""
+    from binade_b200.cuda import kernels as ck
+    from binade_b200.cuda import r4
+
+    g = torch.Generator(device="cuda").manual_seed(N + int(100 * share))
+    out = torch.rand((N, K), generator=g, device="cuda") < share
+    e = torch.where(out, torch.randint(100, 140, (N, K), generator=g, device="cuda"), torch.randint(118, 122, (N, K), generator=g, device="cuda"))
+    w = ((e << 7) | torch.randint(0, 128, (N, K), generator=g, device="cuda")).to(torch.int16).view(torch.bfloat16)
+    m = r4.R4Linear(r4.from_dense(w))
+    x = torch.randn((144, K), generator=g, device="cuda").to(torch.bfloat16)
+    for M in (2, 4, 8):
+        got = words(m.fused_rows(x[:M]))
+        for i in range(M):
+            assert np.array_equal(got[i], words(m(x[i]))), (M, i)
+    half = N // 2 // 4 * 4
+    plain = dict({k: v for k, v in m._a.items() if k not in ("esc_cols", "col_esc")}, raw=m._a["raw"][:half])
+    for M in (17, 144):
+        assert np.array_equal(words(m.mma_rows(x[:M])[:, :half]), words(ck.r4_mma(plain, x[:M], half, K)))
+
+
 @pytest.mark.parametrize("N,K", [(384, 1024), (520, 3840), (256, 15360), (128, 16384)])
 def test_mma_rows_in_the_order_of_cublas(N, K):
     """Split-K in the kernel (every slice from zero in its own accumulator, fp32 sums added in
