@@ -34,18 +34,33 @@ def weights(rng, shape, scale=0.02, escapes=True):
     return u
 
 
-def launches(f) -> int:
-    """Kernel launches of a call, counted as nodes of its CUDA graph."""
-    from cuda.bindings import runtime
+def captured(f) -> list:
+    """The kernel launches of a call as (name, blocks, threads, shared bytes), in no particular order:
+    the nodes of its CUDA graph."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1:]
 
     f()
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         f()
-    status, _, count = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
-    assert status == runtime.cudaError_t.cudaSuccess
-    return count
+    handle = driver.CUgraph(graph.raw_cuda_graph())
+    nodes = ok(driver.cuGraphGetNodes(handle, ok(driver.cuGraphGetNodes(handle, 0))[-1]))[0]
+    out = []
+    for node in nodes:
+        if ok(driver.cuGraphNodeGetType(node))[0] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            p = ok(driver.cuGraphKernelNodeGetParams(node))[0]
+            name = ok(driver.cuFuncGetName(p.func))[0]
+            out.append((name.decode() if isinstance(name, bytes) else str(name), p.gridDimX, p.blockDimX, p.sharedMemBytes))
+    return out
+
+
+def launches(f) -> int:
+    return len(captured(f))
 
 
 def words(t: torch.Tensor) -> np.ndarray:
@@ -261,9 +276,8 @@ def test_transcode_matches_oracle(N, K):
 
 @pytest.mark.parametrize("N,K,kind", [(7201, 260, "normal"), (3601, 132, "normal"), (7107, 4, "normal"), (3553, 3840, "normal"), (7300, 512, "uniform"), (3700, 384, "uniform"), (7200, 640, "mixed"), (3602, 1000, "mixed"), (7110, 128, "const")])
 def test_transcode_many_rows(N, K, kind):
-    """Row counts at which the expander runs four (N >= 7104) or two (N >= 3552) rows a warp:
-    the arrays against the oracle, for short last tiles, a row count that leaves the last warp
-    partly empty, uniformly random words (nearly every weight escapes, every plane count up to the
+    """Thousands of rows, several of them to a warp where they are short: the arrays against the
+    oracle, for short last tiles, a row count that leaves the last warp partly empty, uniformly random words (nearly every weight escapes, every plane count up to the
     format's largest), a mix of both by row, and a constant tensor (no unary plane at all)."""
     from binade_b200.cuda import r4
 
@@ -381,7 +395,6 @@ def test_encode_spreads_short_rows(N, K):
     them, and the arrays are the host encoder's either way (around one row a warp, several rows a
     task, a task cut short)."""
     from binade_b200.cuda import kernels as ck
-    from cuda.bindings import driver
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     u = np.random.default_rng(N + K).integers(0, 1 << 16, (N, K)).astype(np.uint16)
@@ -389,14 +402,7 @@ def test_encode_spreads_short_rows(N, K):
     w, rank = dev(u), torch.arange(256, dtype=torch.uint8, device="cuda")
     meta, words_a_row, roff, total = (torch.empty(n, dtype=t, device="cuda") for n, t in ((N * T, torch.uint8), (N, torch.int32), (N, torch.int32), (1, torch.int64)))
     plan = lambda: ck._call("bn_rice_encode_plan", ck._p(w), ck._p(rank), N, K, ck._p(meta), ck._p(words_a_row), ck._p(roff), ck._p(total))  # noqa: E731
-    plan()
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph):
-        plan()
-    status, nodes, _ = driver.cuGraphGetNodes(driver.CUgraph(graph.raw_cuda_graph()), 2)
-    assert status == driver.CUresult.CUDA_SUCCESS
-    status, params = driver.cuGraphKernelNodeGetParams(nodes[0])
-    assert status == driver.CUresult.CUDA_SUCCESS and params.gridDimX == min(N, sms)
+    assert {n for name, n, _, _ in captured(plan) if "plan_kernel" in name} == {min(N, sms)}
     enc = ck.rice_encode(w)
     for key in ("table", "meta", "bits", "roff"):
         assert np.array_equal(enc[key].cpu().numpy().view(p[key].dtype).reshape(-1), p[key].reshape(-1)), key
@@ -1083,42 +1089,39 @@ def test_mma_waves(rows, M, waves):
     unless the faster decode makes up for it; the product's bits either way."""
     from binade_b200.cuda import kernels as ck
     from binade_b200.cuda import r4
-    from cuda.bindings import driver
-
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     N, K = sms * rows, 128
     g = torch.Generator(device="cuda").manual_seed(rows + M)
     m = r4.R4Linear(r4.from_dense((torch.randn((N, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)))
     x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
     got = m.mma_rows(x)
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph):
-        m.mma_rows(x)
-    status, nodes, _ = driver.cuGraphGetNodes(driver.CUgraph(graph.raw_cuda_graph()), 1)
-    assert status == driver.CUresult.CUDA_SUCCESS
-    status, params = driver.cuGraphKernelNodeGetParams(nodes[0])
-    assert status == driver.CUresult.CUDA_SUCCESS
-    assert -(-params.gridDimX // sms) == waves
+    ((name, blocks, _, shared),) = captured(lambda: m.mma_rows(x))
+    assert -(-blocks // sms) == waves
+    if rows == 104 and "oct" in name:  # two stages of 128 rows of A and of M rows of X beside 40 KB of rings and the 32 KB table
+        assert shared >= 2 * (128 + M) * 256 + 72 * 1024
     half = N // 2  # blocks of other rows, and of the other kernel where those are one wave
     part = {k: (v[:half] if v.dim() > 1 else v) for k, v in m._a.items() if k in ("raw",)}
     top = dict(m._a, raw=part["raw"], codes=m._a["codes"][: half * 32], flags=m._a["flags"][:half], row_esc=m._a["row_esc"][:half], col_esc=m._a["col_esc"][:half])
     assert np.array_equal(words(ck.r4_mma(top, x, half, K)), words(got[:, :half]))
 
 
-@pytest.mark.parametrize("N,K,share", [(4096, 640, 0.1), (4096, 640, 0.9), (8200, 656, 0.6), (15360, 640, 0.45), (15360, 640, 0.55), (15360, 640, 0.95)])
-def test_products_of_escapes(N, K, share):
-    """Weights of which a tenth to nearly all escape, on either side of the lines where products go
-    to the kernels that share a row's escapes among lanes: two to eight rows have the bits of the one-row
-    kernel, the tensor-core product those of row-ordered escapes on another shape."""
+@pytest.mark.parametrize("N,K,share,ways", [(4096, 640, 0.1, "oct oct oct"), (4096, 640, 0.9, "stream stream oct"), (8200, 656, 0.75, "stream stream mma_kernel"), (15360, 640, 0.5, "oct oct oct"), (15360, 640, 0.75, "oct stream mma_kernel")])
+def test_products_of_escapes(N, K, share, ways):
+    """Weights of which a tenth to nearly all escape, on either side of the lines where products (two
+    and eight rows, 144 rows on tensor cores) go to the kernels that share a row's escapes among lanes: two
+    to eight rows have the bits of the one-row kernel, the tensor-core product those of row-ordered
+    escapes on another shape."""
     from binade_b200.cuda import kernels as ck
     from binade_b200.cuda import r4
 
     g = torch.Generator(device="cuda").manual_seed(N + int(100 * share))
     out = torch.rand((N, K), generator=g, device="cuda") < share
-    e = torch.where(out, torch.randint(100, 140, (N, K), generator=g, device="cuda"), torch.randint(118, 122, (N, K), generator=g, device="cuda"))
+    e = torch.where(out, torch.randint(90, 154, (N, K), generator=g, device="cuda"), torch.randint(118, 122, (N, K), generator=g, device="cuda"))
     w = ((e << 7) | torch.randint(0, 128, (N, K), generator=g, device="cuda")).to(torch.int16).view(torch.bfloat16)
     m = r4.R4Linear(r4.from_dense(w))
     x = torch.randn((144, K), generator=g, device="cuda").to(torch.bfloat16)
+    for call, way in zip((lambda: m.fused_rows(x[:2]), lambda: m.fused_rows(x[:8]), lambda: m.mma_rows(x)), ways.split()):
+        assert all(way in name for name, _, _, _ in captured(call)), way
     for M in (2, 4, 8):
         got = words(m.fused_rows(x[:M]))
         for i in range(M):
@@ -1127,6 +1130,26 @@ def test_products_of_escapes(N, K, share):
     plain = dict({k: v for k, v in m._a.items() if k not in ("esc_cols", "col_esc")}, raw=m._a["raw"][:half])
     for M in (17, 144):
         assert np.array_equal(words(m.mma_rows(x[:M])[:, :half]), words(ck.r4_mma(plain, x[:M], half, K)))
+
+
+@pytest.mark.parametrize("rows,K,blocks_an_sm", [(3, 640, 1), (26, 144, 2), (104, 256, 2), (108, 256, 3), (156, 400, 3), (157, 256, 2), (220, 128, 3)])
+def test_decode_blocks(rows, K, blocks_an_sm):
+    """The dense decode's blocks: three an SM only where the weight rows (`rows` an SM and a few more) then
+    take fewer rounds, never fewer than eight warps to build the table; every weight comes back."""
+    from binade_b200.cuda import r4
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(rows + K)
+    w = torch.randn((sms * rows - 5, K), generator=g, device="cuda") * 0.02
+    w = torch.where(torch.rand(w.shape, generator=g, device="cuda") < 0.02, w * 64, w).to(torch.bfloat16)
+    m = r4.R4Linear(r4.from_dense(w))
+    assert np.array_equal(words(m.dense()), words(w))
+    ((_, blocks, threads, _),) = captured(m.dense)
+    assert threads >= 256 and -(-blocks // sms) == blocks_an_sm
+    plain = r4.R4Linear({k: v for k, v in m._a.items() if k not in ("esc_cols", "col_esc")})
+    for key in ("esc_cols", "col_esc"):
+        plain._a.pop(key)
+    assert np.array_equal(words(plain.dense()), words(w))
 
 
 @pytest.mark.parametrize("N,K", [(384, 1024), (520, 3840), (256, 15360), (128, 16384)])
