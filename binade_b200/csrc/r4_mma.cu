@@ -90,9 +90,10 @@ __device__ __forceinline__ bool mm_bar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// True in one lane of the warp, all of which has to get here, whatever its lanes' waits came to. Instructions that a single thread issues (MMAs, commits,
-// bulk copies) take their operands from uniform registers; behind `lane == 0` the compiler has to
-// assume divergent values and wraps each of them in code that makes them uniform.
+// True in one lane of the warp, all of which has to get here: ahead of any wait. Instructions that
+// a single thread issues (MMAs, commits, bulk copies) take their operands from uniform registers;
+// behind `lane == 0` the compiler has to assume divergent values and wraps each of them in code that
+// makes them uniform.
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile(
@@ -592,13 +593,13 @@ __global__ void __launch_bounds__((MAXW + 2) * 32, 1) r4_mma_oct_kernel(const __
     // whether the next stage is there already: asked before the MMAs are issued (which takes as
     // long as the tensor core needs for them), since the answer alone takes more than a hundred cycles
     bool have = false;
-    for (int t = 0; t < T; t++) {  // to the end in every lane, also when its wait gave up: elect.sync takes the whole warp (a vote on the waits cost 1 to 2 us a launch)
+    const bool lead = elect_one();  // here, where the warp is together: its lanes' waits may give up one by one
+    for (int t = 0; t < T; t++) {
       if (ok && !have) ok = mm_bar_wait(win.full + 8 * s, ph);
       const int ns = s + 1 == S ? 0 : s + 1;
       const uint32_t nph = ns ? ph : ph ^ 1u;
       have = mm_bar_test(win.full + 8 * ns, nph);
       tc_fence_after();
-      const bool lead = elect_one();
       if (lead && ok) {
         const uint64_t da = smem_desc(a_at + (uint32_t)s * a_stage), db = smem_desc(b_at + (uint32_t)s * b_stage);
 #pragma unroll
@@ -610,7 +611,6 @@ __global__ void __launch_bounds__((MAXW + 2) * 32, 1) r4_mma_oct_kernel(const __
       s = ns, ph = nph;
       if (++in_slice == a.slice_tiles) in_slice = 0, acc += (uint32_t)a.BN;
     }
-    const bool lead = elect_one();
     if (lead && ok) mma_commit(win.done);
     __syncwarp();
   } else if (x_warp) {
