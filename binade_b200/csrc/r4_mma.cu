@@ -137,7 +137,7 @@ struct MmaArgs {
   uint16_t *y;
   int64_t N, K, y_stride;
   int T, M, BN, stages;
-  int rows;  // weight rows per block (a multiple of MMA_RPW, at most MMA_ROWS)
+  int rows;  // weight rows per block: a multiple of four up to 104 (eight threads per row), else of MMA_RPW up to 112
   uint32_t tmem_cols;
   // split-K as cuBLAS does it for few input rows and long K: `split` equal slices of the K tiles,
   // each summed from zero into its own accumulator (BN columns apart in tensor memory), the
@@ -385,7 +385,6 @@ struct MmaOctPlan {
   int phases, groups;   // tile phases; row groups of four (groups * phases decode warps)
   int a_rows;           // rows of an A stage: the block's, rounded up to 8, or 128
   int m;                // MMA M: 64 for up to 64 rows (half the A bytes to read per MMA, which is what few input rows cost), else 128
-  int slots;            // stages
   uint32_t ring_slot;   // bytes of a warp's ring slot: 512 raw, 256 codes, 256 for the codes of each skipped tile
   uint32_t flag_words;  // words of a row's flag bits in shared memory, a zero word in front
 };

@@ -6,8 +6,10 @@
 //   x        M rows as BF16 in shared memory, in the unused halves of the pair table's entries where
 //            they fit (M T <= 128), else above the table; 32 bytes a thread, tile and row
 //   grouped  blockIdx.y is the i-th group of up to M slots over all experts, found by a prefix sum of
-//            the experts' group counts at block start, so that the grid holds hardly more blocks
-//            than there is work; blocks of one group share an expert's rows (grid.x)
+//            the experts' group counts at block start; the grid holds the most groups there can be
+//            (active experts + slots / M: 256 for the about 176 groups of 64 tokens, top 8 of 128),
+//            and a block past the last group leaves at once; blocks of one group share an expert's
+//            rows (grid.x)
 //   half     a block with at most M / 2 input rows runs the code for M / 2
 //   end of a row  the 4 M accumulators of a thread are summed over the row's eight threads while the
 //            input rows are dealt out to them (16 shuffles instead of 48 for M = 4); additions pair

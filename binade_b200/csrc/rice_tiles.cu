@@ -11,9 +11,12 @@
 //                      bit planes of min(rank, 15) are transposed to nibbles in registers
 //
 // The decoder with a warp per row (rice_kernel) spends a warp-wide step on every plane of every
-// tile, 240 to 500 warp instructions a tile; here 30 tiles share 2300, and the scan adds 49 a tile.
+// tile, 240 to 500 warp instructions a tile; here 30 tiles share 2470, and the scan adds 52 a tile.
 // Measured with the benchmark's distribution (us, warp per row -> here): R4 arrays of 15360 x 3840
-// 192 -> 44 + 68 (scan + tiles), of 3840 x 15360 350 -> 115 + 65; BF16 words of 22528 x 704 97 -> 15 + 44.
+// 192 -> 41 + 63 (scan + tiles), of 3840 x 15360 350 -> 113 + 72; BF16 words of 22528 x 704 97 -> 12 + 36.
+// Escapes cost little while they are few: a tile's last eight weights are at hand, the others come out
+// of one more walk over its planes, and tiles with three low bits, where most weights escape, are
+// decoded one at a time by the whole warp (rice_kernels.cu takes streams that are full of such tiles).
 // The tiles' first bits wait in the output array itself (the last 4 T bytes of each output row):
 // entry t lies in the bytes of tile t or later, and a row's tiles are decoded in order by one
 // warp that reads its entries first, so no entry is overwritten before it is read.
@@ -69,7 +72,7 @@ __device__ __noinline__ uint32_t scan_long_tile(const uint32_t *__restrict__ bit
 // One warp per block, four lanes per row (`rows_per_block` <= 8 rows): a lane counts 32 of up to 128
 // bits of a plane; planes of few bits are counted by all four alike. slots + (row + 1) * row_bytes -
 // 4 (T - t) receives tile t's first bit, counted from the row's first word.
-// Bound: the instructions of a row's chain of dependent counts (345 a step, 54 % of issue slots).
+// Bound: the instructions of a row's chain of dependent counts (366 a step, 57 % of issue slots).
 // With a row per lane the walk takes 537 instructions a step (the slowest of 26 rows decides each
 // loop) in a quarter of the warps: as long on 15360 rows (44 us), longer on fewer.
 template <int MODE>
@@ -225,8 +228,8 @@ __device__ __forceinline__ uint4 nibbles(uint32_t r0, uint32_t r1, uint32_t r2, 
 }
 
 // A warp takes `rows_per_task` whole rows (several when 32 tiles hold them), 32 tiles at a time.
-// Bound: shared memory (60 % of its cycles: the deposit table's conflicts) and issue (59 %). Of the
-// 2300 instructions of a 30-tile row a plane's deposits take 164, about five planes of them; with
+// Bound: shared memory (61 % of its cycles: the deposit table's conflicts) and issue (63 %). Of the
+// 2470 instructions of a 30-tile row a plane's deposits take 164, about five planes of them; with
 // the last few weights of a plane taken one by one instead of as one more deposit the kernel took
 // 95 us on 15360 x 3840.
 template <int MODE>

@@ -27,7 +27,11 @@ from torch import nn
 from ..format import TILE
 from . import kernels as ck
 
-FUSED_MAX_ROWS = 4  # input rows served by the fused decode kernel in the documented order (15360 x 3840: 23 / 33 / 53 us at 2 / 4 / 8 rows); from 5 rows the tensor-core decode GEMM is faster (33 us)
+# Input rows served by the fused decode kernel in the documented order. Us at 2 / 4 / 8 rows and, from five
+# rows, the tensor-core decode GEMM: 15360 x 3840 25 / 33 / 52 and 34, 4096 x 3840 13 / 16 / 21 and 19. Rows of
+# 15360 columns do not fit in one pass (3840 x 15360 41 / 82 / 169 and 54): there the documented order up to
+# four rows has its price.
+FUSED_MAX_ROWS = 4
 
 
 MMA_MAX_ROWS = 256  # input rows served by the tensor-core decode GEMM (one pass over the weights; 256 is the MMA's widest N); beyond, rebuild + cuBLAS
