@@ -421,7 +421,7 @@ def some_heavy_tiles(rng, N, K):
 @pytest.mark.parametrize("N,K", [(33001, 4), (17001, 132), (11003, 260), (70, 1000), (33, 2048), (9, 2052), (40, 4096), (11, 4100), (3, 12296)])
 def test_thread_per_tile_escapes(N, K):
     """Tiles of every k with many escapes among ordinary ones, 1 to 97 tiles a row: file arrays, BF16
-    rows and R4 arrays (each alone would be a stream for the decoder with a warp per row)."""
+    rows, looked-up rows and R4 arrays (each alone would be a stream for the decoder with a warp per row)."""
     from binade_b200.cuda import kernels as ck
     from binade_b200.cuda import r4
 
@@ -438,6 +438,9 @@ def test_thread_per_tile_escapes(N, K):
     out, rend = ck.rice_unpack(d["meta"].reshape(-1), d["bits"], d["roff"], d["table"], d["raw"], N, K)
     assert np.array_equal(words(out), u)
     assert np.array_equal(rend.cpu().numpy().view(np.uint32), np.append(p["roff"][1:], np.uint32(len(p["bits"]))))
+    ids = np.array([N - 1, 0, N, N // 2, 0] * 40, np.int32)
+    rows = words(ck.rice_lookup(d["meta"].reshape(-1), d["bits"], d["roff"], d["table"], d["raw"], N, K, ck.to_device(ids)))
+    assert np.array_equal(rows, np.where((ids < N)[:, None], u[np.minimum(ids, N - 1)], np.uint16(0)))
 
 
 @pytest.mark.parametrize("N,K", [(64, 2048), (2048, 1024), (30000, 128)])
