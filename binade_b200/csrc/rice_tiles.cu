@@ -125,9 +125,7 @@ __global__ void __launch_bounds__(32) rice_scan_kernel(RiceArgs a, uint8_t *slot
       const uint32_t n = (uint32_t)min((int64_t)BN_TILE, a.K - (int64_t)t * BN_TILE);
       const uint32_t most = n * (k + qmax);
       const bool is_long = most > SC_BLOCK * 32u;
-      // (a long tile starts with both blocks of the ring at hand)
-      const uint32_t need = min(most, 2u * SC_BLOCK * 32u - (cur & (SC_BLOCK * 32u - 1u)));
-      const bool go = t < T && cur + need <= usable * (SC_BLOCK * 32u);
+      const bool go = t < T && cur + min(most, SC_BLOCK * 32u) <= usable * (SC_BLOCK * 32u);  // (a long tile starts with a block's length of bits at hand)
       if (!__any_sync(BN_FULL, go)) break;
       if (go) {
         if (part == 0) slot[t] = cur - off;
